@@ -11,75 +11,126 @@
 namespace tn {
 
 // ------------------------------------------------------------------------------------
-// grouped GEMM: one CTA per 64x64 output tile, 256 threads, 4x4 outputs per thread
+// grouped GEMM: 128 threads per TM x TN output tile, one thread adds its outputs along the
+// whole k range of the task
+//
+// Bound by the FP64 pipe: a warp-wide DFMA holds its SM sub-partition for 64 clocks (measured:
+// 1.7 FMA per clock and SM with one warp per sub-partition, 2.0 at most; DMMA the same), so a
+// multiplication by padding costs as much as a real one, while loads, shared memory and issue
+// slots are nearly free.  Hence small tiles of 8 x 4 warp patches (patches outside the block
+// are skipped), k taken to its exact end, the segments of a task run together into one k range
+// (four 4-long segments fill a 16-deep chunk), four warps so that every sub-partition works,
+// and the next chunk's loads in flight during the products.  Each output is one chain of fused
+// multiply-adds in segment order.  On the 64 x 64 x 16 tiles of 256 threads that this replaced
+// a 4 x 4 x 4 block took 16 us of multiplications by zeros.
+// The tile is GemmPlan::finalize's choice.  Measured, whole calls in FP64: DMRG run of a
+// 12-site chain 118 -> 71 ms, sweep of a 20-site cylinder at chi = 160 236 -> 95 ms, TDVP of
+// a 12-site chain (complex) 209 -> 91 ms, sweep of a 16-site tree at chi = 16 75 -> 41 ms.
 // ------------------------------------------------------------------------------------
 namespace {
 constexpr int BK = 16;
+constexpr int GEMM_THREADS = 128;
 
-__global__ void __launch_bounds__(256)
+template <int TM, int TN>
+__global__ void __launch_bounds__(GEMM_THREADS)
 gemm_f64_kernel(const Seg* __restrict__ segs, const Task* __restrict__ tasks,
-                const Tile* __restrict__ tiles, Bases b) {
-    __shared__ double As[BK][GEMM_BM + 1];
-    __shared__ double Bs[BK][GEMM_BN + 1];
+                const Tile* __restrict__ tiles, const __grid_constant__ Bases b) {
+    constexpr int RP = TM / 16, CP = TN / 8;          // 8-row and 4-column patches of a warp
+    constexpr int NA = TM * BK / GEMM_THREADS, NB = TN * BK / GEMM_THREADS;  // loads per thread
+    __shared__ double As[BK][TM + 1];
+    __shared__ double Bs[BK][TN + 1];
     const Tile t = tiles[blockIdx.x];
     const Task tk = tasks[t.task];
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    double acc[4][4];
+    const Seg* const seg0 = segs + tk.seg0;
+    const int K = tk.nseg ? seg0[tk.nseg - 1].kpre + seg0[tk.nseg - 1].k : 0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row0 = (warp & 1) * (TM / 2) + (lane & 7);
+    const int col0 = (warp >> 1) * (TN / 2) + (lane >> 3);
+    // rows and columns of the block from this warp's first patch on
+    const int mrem = tk.m - t.m0 - (warp & 1) * (TM / 2);
+    const int nrem = tk.n - t.n0 - (warp >> 1) * (TN / 2);
+    double acc[RP][CP];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RP; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
+        for (int j = 0; j < CP; ++j) acc[i][j] = 0.0;
 
-    for (int si = 0; si < tk.nseg; ++si) {
-        const Seg sg = segs[tk.seg0 + si];
-        const double* __restrict__ A = b.p[sg.abuf] + sg.aoff;
-        const double* __restrict__ B = b.p[sg.bbuf] + sg.boff;
-        for (int k0 = 0; k0 < sg.k; k0 += BK) {
-            for (int e = tid; e < GEMM_BM * BK; e += 256) {
-                int i, kk;
-                if (!sg.ta) { i = e % GEMM_BM; kk = e / GEMM_BM; }
-                else        { kk = e % BK; i = e / BK; }
-                const int gi = t.m0 + i, gk = k0 + kk;
+    if (K > 0) {
+        // element order of the loads: along the operand's contiguous index (as the first
+        // segment has it; the others of a task are alike)
+        const bool ka = seg0->ta != 0, kb = seg0->tb == 0;  // k is the contiguous index
+        const Seg *wa = seg0, *wb = seg0;  // segments of this thread's last loads
+        double ra[NA], rb[NB];
+        auto load = [&](int k0) {
+#pragma unroll
+            for (int r = 0; r < NA; ++r) {
+                const int e = tid + GEMM_THREADS * r;
+                const int i = t.m0 + (ka ? e / BK : e % TM);
+                const int kf = k0 + (ka ? e % BK : e / TM);
                 double v = 0.0;
-                if (gi < tk.m && gk < sg.k)
-                    v = sg.ta ? A[gk + int64_t(gi) * sg.lda] : A[gi + int64_t(gk) * sg.lda];
-                As[kk][i] = sg.sgn < 0 ? -v : v;
+                if (kf < K && i < tk.m) {
+                    while (kf >= wa->kpre + wa->k) ++wa;
+                    const double* A = b.p[wa->abuf] + wa->aoff;
+                    const int64_t k = kf - wa->kpre;
+                    v = wa->ta ? A[k + int64_t(i) * wa->lda] : A[i + k * wa->lda];
+                    v = wa->sgn < 0 ? -v : v;
+                }
+                ra[r] = v;
             }
-            for (int e = tid; e < GEMM_BN * BK; e += 256) {
-                int j, kk;
-                if (!sg.tb) { kk = e % BK; j = e / BK; }
-                else        { j = e % GEMM_BN; kk = e / GEMM_BN; }
-                const int gj = t.n0 + j, gk = k0 + kk;
+#pragma unroll
+            for (int r = 0; r < NB; ++r) {
+                const int e = tid + GEMM_THREADS * r;
+                const int j = t.n0 + (kb ? e / BK : e % TN);
+                const int kf = k0 + (kb ? e % BK : e / TN);
                 double v = 0.0;
-                if (gj < tk.n && gk < sg.k)
-                    v = sg.tb ? B[gj + int64_t(gk) * sg.ldb] : B[gk + int64_t(gj) * sg.ldb];
-                Bs[kk][j] = v;
+                if (kf < K && j < tk.n) {
+                    while (kf >= wb->kpre + wb->k) ++wb;
+                    const double* B = b.p[wb->bbuf] + wb->boff;
+                    const int64_t k = kf - wb->kpre;
+                    v = wb->tb ? B[j + k * wb->ldb] : B[k + int64_t(j) * wb->ldb];
+                }
+                rb[r] = v;
+            }
+        };
+        load(0);
+        for (int k0 = 0; k0 < K; k0 += BK) {
+#pragma unroll
+            for (int r = 0; r < NA; ++r) {
+                const int e = tid + GEMM_THREADS * r;
+                As[ka ? e % BK : e / TM][ka ? e / BK : e % TM] = ra[r];
+            }
+#pragma unroll
+            for (int r = 0; r < NB; ++r) {
+                const int e = tid + GEMM_THREADS * r;
+                Bs[kb ? e % BK : e / TN][kb ? e / BK : e % TN] = rb[r];
             }
             __syncthreads();
+            if (k0 + BK < K) load(k0 + BK);
+            const int kv = min(BK, K - k0);
+#pragma unroll 4
+            for (int kk = 0; kk < kv; ++kk) {
+                double a[RP], q[CP];
 #pragma unroll
-            for (int kk = 0; kk < BK; ++kk) {
-                double a[4], bb[4];
+                for (int i = 0; i < RP; ++i) a[i] = As[kk][row0 + 8 * i];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] = As[kk][tx + 16 * i];
+                for (int j = 0; j < CP; ++j) q[j] = Bs[kk][col0 + 4 * j];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) bb[j] = Bs[kk][ty + 16 * j];
+                for (int i = 0; i < RP; ++i)
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], bb[j], acc[i][j]);
+                    for (int j = 0; j < CP; ++j)
+                        if (8 * i < mrem && 4 * j < nrem) acc[i][j] = fma(a[i], q[j], acc[i][j]);
             }
             __syncthreads();
         }
     }
     double* __restrict__ C = b.p[tk.cbuf] + tk.coff;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int gj = t.n0 + ty + 16 * j;
+    for (int j = 0; j < CP; ++j) {
+        const int gj = t.n0 + col0 + 4 * j;
         if (gj >= tk.n) continue;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int gi = t.m0 + tx + 16 * i;
+        for (int i = 0; i < RP; ++i) {
+            const int gi = t.m0 + row0 + 8 * i;
             if (gi < tk.m) {
                 double* c = C + gi + int64_t(gj) * tk.ldc;
                 *c = tk.accum ? *c + acc[i][j] : acc[i][j];
@@ -308,7 +359,10 @@ VecPtrs make_ptrs(const double* const* V, int K) {
 
 void launch_gemm_f64(const GemmPlan& p, const Bases& b, cudaStream_t s) {
     if (p.tiles.empty()) return;
-    gemm_f64_kernel<<<unsigned(p.tiles.size()), 256, 0, s>>>(
+    auto* kernel = p.tile_n == 32   ? gemm_f64_kernel<32, 32>
+                   : p.tile_n == 16 ? gemm_f64_kernel<16, 16>
+                                    : gemm_f64_kernel<16, 8>;
+    kernel<<<unsigned(p.tiles.size()), GEMM_THREADS, 0, s>>>(
         p.dsegs.as<Seg>(), p.dtasks.as<Task>(), p.dtiles.as<Tile>(), b);
     TN_CUDA(cudaGetLastError());
     count_launch();

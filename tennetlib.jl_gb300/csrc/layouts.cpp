@@ -202,8 +202,10 @@ void GemmPlan::add_seg(int abuf, int64_t aoff, int lda, int ta, int bbuf, int64_
     s.k = k;
     s.ta = ta;
     s.tb = tb;
-    segs.push_back(s);
     Task& t = tasks.back();
+    s.kpre = t.nseg ? segs.back().kpre + segs.back().k : 0;
+    s.pad = 0;
+    segs.push_back(s);
     t.nseg += 1;
     flops += 2.0 * double(t.m) * double(t.n) * double(k);
 }
@@ -220,19 +222,43 @@ void GemmPlan::finalize(cudaStream_t s) {
     tiles.clear();
     // heavy tasks first so that the tail of the grid is made of small tiles
     std::vector<int> order(tasks.size());
-    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
-    auto work = [&](int i) {
-        double k = 0;
-        for (int j = 0; j < tasks[i].nseg; ++j) k += segs[tasks[i].seg0 + j].k;
-        return k;
-    };
     std::vector<double> w(tasks.size());
-    for (size_t i = 0; i < tasks.size(); ++i) w[i] = work((int)i);
+    for (size_t i = 0; i < order.size(); ++i) {
+        order[i] = (int)i;
+        const Task& t = tasks[i];
+        w[i] = t.nseg ? double(segs[size_t(t.seg0 + t.nseg - 1)].kpre) +
+                            segs[size_t(t.seg0 + t.nseg - 1)].k
+                      : 0.0;
+    }
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return w[a] > w[b]; });
+    // Output tile by the estimated time of the launch, in clocks: every 8 x 4 patch and k
+    // holds the FP64 pipe of its SM for 16 clocks (64 on one of four sub-partitions), so a
+    // launch takes at least the total over the SMs and at least its longest tile.  Small plans
+    // are bound by the longest tile (a 90 x 45 block with k = 900: 64, 128 or 512 clocks per k
+    // on 16 x 8, 16 x 16 or 32 x 32), large ones by the total, where 32 x 32 has fewer CTAs.
+    constexpr double SMS = 152.0, CTA = 1200.0;
+    constexpr int TILES[3][2] = {{32, 32}, {16, 16}, {16, 8}};
+    double best = -1.0;
+    for (const auto& T : TILES) {
+        double total = 0.0, ntile = 0.0, longest = 0.0;
+        for (size_t i = 0; i < tasks.size(); ++i) {
+            const Task& t = tasks[i];
+            const int pm = (t.m + 7) / 8, pn = (t.n + 3) / 4;
+            total += 16.0 * pm * pn * w[i];
+            ntile += double((t.m + T[0] - 1) / T[0]) * ((t.n + T[1] - 1) / T[1]);
+            longest = std::max(longest, 64.0 * std::min(pm, T[0] / 16) * std::min(pn, T[1] / 8) * w[i]);
+        }
+        const double est = std::max((total + CTA * ntile) / SMS, longest + CTA);
+        if (best < 0.0 || est < best) {
+            best = est;
+            tile_m = T[0];
+            tile_n = T[1];
+        }
+    }
     for (int ti : order) {
         const Task& t = tasks[ti];
-        for (int m0 = 0; m0 < t.m; m0 += GEMM_BM)
-            for (int n0 = 0; n0 < t.n; n0 += GEMM_BN) tiles.push_back(Tile{ti, m0, n0});
+        for (int m0 = 0; m0 < t.m; m0 += tile_m)
+            for (int n0 = 0; n0 < t.n; n0 += tile_n) tiles.push_back(Tile{ti, m0, n0});
     }
     upload(dsegs, segs, s);
     upload(dtasks, tasks, s);

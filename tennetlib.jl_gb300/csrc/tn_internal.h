@@ -141,6 +141,7 @@ struct Bases {
 struct Seg {
     int64_t aoff, boff;
     int32_t abuf, bbuf, lda, ldb, k, ta, tb, sgn;
+    int32_t kpre, pad;  // k of the task's earlier segments
 };
 struct Task {
     int64_t coff;
@@ -169,6 +170,7 @@ struct GemmPlan {
     std::vector<Task> tasks;
     std::vector<Tile> tiles;
     double flops = 0;
+    int tile_m = 32, tile_n = 32;  // output tile of the FP64 kernel
     DevBuf dsegs, dtasks, dtiles;
     void add_task(int cbuf, int64_t coff, int m, int n, int ldc, int accum = 0);
     void add_seg(int abuf, int64_t aoff, int lda, int ta, int bbuf, int64_t boff, int ldb,
@@ -238,7 +240,6 @@ void launch_split_gemm(const SplitItem* items, int nitems, const SplitTask* task
                        const uint8_t* apack, const uint8_t* bpack, const int* ea, const int* eb,
                        const Bases& b, int slices, int* err, int nsm, cudaStream_t s);
 
-constexpr int GEMM_BM = 64, GEMM_BN = 64;
 constexpr int COMB_TR = 32, COMB_TC = 32;
 
 // ------------------------------------------------------------------------------------
