@@ -1170,11 +1170,7 @@ EigOut lanczos_lowest(tn_env* env, MV&& apply, int64_t n, double* x0, double* re
     env->kry.alloc(size_t(nvec) * size_t(std::max<int64_t>(n, 1)) * 8, st);
     env->part.alloc(size_t(32) * blas_nparts() * 8, st);
     env->dots.alloc(128 * 8, st);
-    if (!env->ticket.p) {
-        env->ticket.alloc(sizeof(unsigned), st);
-        TN_CUDA(cudaMemsetAsync(env->ticket.p, 0, sizeof(unsigned), st));
-    }
-    unsigned* tk = env->ticket.as<unsigned>();
+    unsigned* tk = ctx->gs_ticket.as<unsigned>();
     std::vector<double*> pool;
     for (int i = 0; i < nvec; ++i) pool.push_back(env->kry.d() + int64_t(i) * n);
     double* dv = env->dots.d();
@@ -1188,32 +1184,30 @@ EigOut lanczos_lowest(tn_env* env, MV&& apply, int64_t n, double* x0, double* re
         return q;
     };
     EigOut out{0.0, 0, 0};
-    std::vector<double> hostd(65);
 
+    // h = V^T w ; w -= V h ; twice ; beta = |w| ; the next basis vector w / beta is formed on
+    // the way while the Krylov space still grows (into the slot that take() hands out next)
+    double start2 = 0.0;  // squared norm of x0, known from the first step on
+    double* ready = nullptr;
     auto gs2 = [&](int K, std::vector<double>& h, double& beta) {
-        // h = V^T w ; w -= V h ; twice ; beta = |w|
+        ready = K < kd ? pool.back() : nullptr;
         const int e0 = ctx->timer.mark();
-        launch_gs_pass(V.data(), K, w, nullptr, 0.0, n, true, false, env->part.d(), dv, tk, st);
-        launch_gs_pass(V.data(), K, w, dv, -1.0, n, true, false, env->part.d(), dv + 32, tk, st);
-        launch_gs_pass(V.data(), K, w, dv + 32, -1.0, n, false, true, env->part.d(), dv + 64, tk, st);
+        launch_gs2(V.data(), K, w, ready, n, env->part.d(), dv, tk, ctx->post.next(dv + GS_START),
+                   st);
         ctx->timer.add(T_LANCZOS, e0, ctx->timer.mark());
-        TN_CUDA(cudaMemcpyAsync(hostd.data(), dv, 65 * 8, cudaMemcpyDeviceToHost, st));
-        sync(ctx);
+        const double* r = ctx->post.wait(st);
         h.resize(K);
-        for (int i = 0; i < K; ++i) h[i] = hostd[i] + hostd[32 + i];
-        beta = std::sqrt(std::max(hostd[64], 0.0));
+        for (int i = 0; i < K; ++i) h[i] = r[i] + r[GS_H2 + i];
+        beta = std::sqrt(std::max(r[GS_NORM], 0.0));
+        start2 = r[GS_START];
     };
 
     // normalise x0 into V[0]
     {
         const double* xp = x0;
-        launch_multi_dot(&xp, 1, x0, n, env->part.d(), dv + 64, st);
-        double nrm2 = 0;
-        TN_CUDA(cudaMemcpyAsync(&nrm2, dv + 64, 8, cudaMemcpyDeviceToHost, st));
-        sync(ctx);
-        TN_REQUIRE(nrm2 > 0.0, "eigensolver start vector is zero");
+        launch_multi_dot(&xp, 1, x0, n, env->part.d(), dv + GS_START, tk, st);
         double* v0 = take();
-        launch_scale_into(v0, x0, nullptr, 1.0 / std::sqrt(nrm2), n, st);
+        launch_scale_into(v0, x0, dv + GS_START, 1.0, n, st);
         V.push_back(v0);
     }
     std::vector<double> Hm(size_t(kd + 1) * (kd + 1), 0.0);
@@ -1223,6 +1217,7 @@ EigOut lanczos_lowest(tn_env* env, MV&& apply, int64_t n, double* x0, double* re
     apply(V[0], w);
     out.matvecs++;
     gs2(1, h, beta);
+    TN_REQUIRE(start2 > 0.0, "eigensolver start vector is zero");
     Hat(0, 0) = h[0];
     int numiter = 1;
     std::vector<double> D, U;
@@ -1243,7 +1238,7 @@ EigOut lanczos_lowest(tn_env* env, MV&& apply, int64_t n, double* x0, double* re
         }
         if (K < kd) {
             double* v = take();
-            launch_scale_into(v, w, nullptr, 1.0 / beta, n, st);
+            if (v != ready) launch_scale_into(v, w, nullptr, 1.0 / beta, n, st);
             V.push_back(v);
             apply(v, w);
             out.matvecs++;
@@ -1256,15 +1251,13 @@ EigOut lanczos_lowest(tn_env* env, MV&& apply, int64_t n, double* x0, double* re
             if (numiter == prm->maxiter) break;
             const int keep = (3 * kd + 2 * converged) / 5;
             std::vector<double*> NV;
+            std::vector<double> coef(size_t(keep) * K);
             for (int j = 0; j < keep; ++j) {
-                double* q = take();
-                std::vector<double> coef(K);
-                for (int i = 0; i < K; ++i) coef[i] = U[size_t(i) * K + j];
-                TN_CUDA(cudaMemcpyAsync(dv + 96, coef.data(), K * 8, cudaMemcpyHostToDevice, st));
-                launch_lincomb(q, V.data(), K, dv + 96, n, st);
-                sync(ctx);  // coef staging slot is reused
-                NV.push_back(q);
+                NV.push_back(take());
+                for (int i = 0; i < K; ++i) coef[size_t(j) * K + i] = U[size_t(i) * K + j];
             }
+            launch_lincomb(NV.data(), keep, V.data(), K, coef.data(), n, st);
+            ready = nullptr;
             for (double* q : V) pool.push_back(q);
             V = NV;
             std::fill(Hm.begin(), Hm.end(), 0.0);
@@ -1276,12 +1269,10 @@ EigOut lanczos_lowest(tn_env* env, MV&& apply, int64_t n, double* x0, double* re
     const int K = (int)V.size();
     std::vector<double> coef(K);
     for (int i = 0; i < K; ++i) coef[i] = U[size_t(i) * K + 0];
-    TN_CUDA(cudaMemcpyAsync(dv + 96, coef.data(), K * 8, cudaMemcpyHostToDevice, st));
-    launch_lincomb(result, V.data(), K, dv + 96, n, st);
+    launch_lincomb(&result, 1, V.data(), K, coef.data(), n, st);
     const double* rp = result;
-    launch_multi_dot(&rp, 1, result, n, env->part.d(), dv + 64, st);
-    launch_scale_into(result, result, dv + 64, 1.0, n, st);
-    sync(ctx);
+    launch_multi_dot(&rp, 1, result, n, env->part.d(), dv + GS_NORM, tk, st);
+    launch_scale_into(result, result, dv + GS_NORM, 1.0, n, st);
     out.energy = D[0];
     out.converged = converged;
     return out;
@@ -1312,11 +1303,7 @@ int krylov_exp(tn_env* env, MV&& apply, int64_t n, double t, const double* x0, d
     env->kry.alloc(size_t(nvec) * size_t(std::max<int64_t>(n, 1)) * 8, st);
     env->part.alloc(size_t(32) * blas_nparts() * 8, st);
     env->dots.alloc(256 * 8, st);
-    if (!env->ticket.p) {
-        env->ticket.alloc(sizeof(unsigned), st);
-        TN_CUDA(cudaMemsetAsync(env->ticket.p, 0, sizeof(unsigned), st));
-    }
-    unsigned* tk = env->ticket.as<unsigned>();
+    unsigned* tk = ctx->gs_ticket.as<unsigned>();
     double* dv = env->dots.d();
     std::vector<double*> pool;
     for (int i = 0; i < nvec; ++i) pool.push_back(env->kry.d() + int64_t(i) * n);
@@ -1325,47 +1312,34 @@ int krylov_exp(tn_env* env, MV&& apply, int64_t n, double t, const double* x0, d
     double* w = pool.back();
     pool.pop_back();
     TN_CUDA(cudaMemcpyAsync(cur, x0, size_t(n) * 8, cudaMemcpyDeviceToDevice, st));
-    std::vector<double> hostd(65);
     int matvecs = 0;
     double rem = 1.0;  // fraction of tau still to go
     const double tabs = std::hypot(t, ti);
-    if (ti != 0.0) {
-        const double one = 1.0;
-        TN_CUDA(cudaMemcpyAsync(dv + 224, &one, 8, cudaMemcpyHostToDevice, st));
-    }
-    auto norm2 = [&](double* v) {
-        const double* vp = v;
-        launch_gs_pass(&vp, 0, v, nullptr, 0.0, n, false, true, env->part.d(), dv + 64, tk, st);
-        double r = 0;
-        TN_CUDA(cudaMemcpyAsync(&r, dv + 64, 8, cudaMemcpyDeviceToHost, st));
-        sync(ctx);
-        return r;
-    };
     for (int it = 0; it < prm->maxiter && rem != 0.0; ++it) {
-        const double nrm = std::sqrt(std::max(norm2(cur), 0.0));
-        if (nrm == 0.0) break;
+        launch_gs_pass(nullptr, 0, cur, nullptr, 0.0, n, true, env->part.d(), dv + GS_START, tk, st);
+        double nrm = 0.0;  // |cur|, known from the first Gram-Schmidt step on
         std::vector<double*> V;
         V.push_back(pool[0]);
-        launch_scale_into(V[0], cur, nullptr, 1.0 / nrm, n, st);
+        launch_scale_into(V[0], cur, dv + GS_START, 1.0, n, st);
         std::vector<double> Hm(size_t(kd + 1) * (kd + 1), 0.0);
         auto Hat = [&](int i, int j) -> double& { return Hm[size_t(i) * (kd + 1) + j]; };
         auto gs = [&](int K, std::vector<double>& h, double& beta) {
             const int e0 = ctx->timer.mark();
-            launch_gs_pass(V.data(), K, w, nullptr, 0.0, n, true, false, env->part.d(), dv, tk, st);
-            launch_gs_pass(V.data(), K, w, dv, -1.0, n, true, false, env->part.d(), dv + 32, tk, st);
-            launch_gs_pass(V.data(), K, w, dv + 32, -1.0, n, false, true, env->part.d(), dv + 64, tk, st);
+            launch_gs2(V.data(), K, w, K < kd ? pool[K] : nullptr, n, env->part.d(), dv, tk,
+                       ctx->post.next(dv + GS_START), st);
             ctx->timer.add(T_LANCZOS, e0, ctx->timer.mark());
-            TN_CUDA(cudaMemcpyAsync(hostd.data(), dv, 65 * 8, cudaMemcpyDeviceToHost, st));
-            sync(ctx);
+            const double* r = ctx->post.wait(st);
             h.resize(K);
-            for (int i = 0; i < K; ++i) h[i] = hostd[i] + hostd[32 + i];
-            beta = std::sqrt(std::max(hostd[64], 0.0));
+            for (int i = 0; i < K; ++i) h[i] = r[i] + r[GS_H2 + i];
+            beta = std::sqrt(std::max(r[GS_NORM], 0.0));
+            nrm = std::sqrt(std::max(r[GS_START], 0.0));
         };
         std::vector<double> h, D, U;
         double beta = 0.0;
         apply(V[0], w);
         matvecs++;
         gs(1, h, beta);
+        if (nrm == 0.0) break;
         Hat(0, 0) = h[0];
         double f = rem;  // this step: tau f
         while (true) {
@@ -1404,26 +1378,17 @@ int krylov_exp(tn_env* env, MV&& apply, int64_t n, double t, const double* x0, d
             }
             if (accept) {
                 for (double& c : yr) c *= nrm;
-                TN_CUDA(cudaMemcpyAsync(dv + 96, yr.data(), K * 8, cudaMemcpyHostToDevice, st));
-                launch_lincomb(cur, V.data(), K, dv + 96, n, st);
                 if (ti != 0.0) {
-                    // cur += i (sum_j Im(y_j) v_j), through the residual buffer
                     for (double& c : yi) c *= nrm;
-                    TN_CUDA(cudaMemcpyAsync(dv + 160, yi.data(), K * 8, cudaMemcpyHostToDevice, st));
-                    launch_lincomb(w, V.data(), K, dv + 160, n, st);
-                    const double* wim = w + nc;
-                    const double* wre = w;
-                    launch_multi_axpy(cur, &wim, 1, dv + 224, -1.0, nc, st);
-                    launch_multi_axpy(cur + nc, &wre, 1, dv + 224, 1.0, nc, st);
+                    launch_lincomb_complex(cur, V.data(), K, yr.data(), yi.data(), nc, st);
+                } else {
+                    launch_lincomb(&cur, 1, V.data(), K, yr.data(), n, st);
                 }
-                sync(ctx);
                 rem -= f;
                 break;
             }
-            double* v = pool[K];
-            launch_scale_into(v, w, nullptr, 1.0 / beta, n, st);
-            V.push_back(v);
-            apply(v, w);
+            V.push_back(pool[K]);  // w / beta, formed by the Gram-Schmidt step
+            apply(V.back(), w);
             matvecs++;
             gs(K + 1, h, beta);
             for (int i = 0; i <= K; ++i) {
@@ -1442,19 +1407,17 @@ double normalize_and_energy(tn_env* env, MV&& apply, int64_t n, double* x, doubl
                             bool normalize) {
     tn_ctx* ctx = env->ctx;
     cudaStream_t st = ctx->stream;
-    unsigned* tk = env->ticket.as<unsigned>();
+    unsigned* tk = ctx->gs_ticket.as<unsigned>();
     double* dv = env->dots.d();
     const double* xp = x;
     if (normalize) {
-        launch_gs_pass(&xp, 0, x, nullptr, 0.0, n, false, true, env->part.d(), dv + 64, tk, st);
-        launch_scale_into(x, x, dv + 64, 1.0, n, st);
+        launch_gs_pass(nullptr, 0, x, nullptr, 0.0, n, true, env->part.d(), dv + GS_NORM, tk, st);
+        launch_scale_into(x, x, dv + GS_NORM, 1.0, n, st);
     }
     apply(x, y);
-    launch_gs_pass(&xp, 1, y, nullptr, 0.0, n, true, false, env->part.d(), dv + 64, tk, st);
-    double e = 0.0;
-    TN_CUDA(cudaMemcpyAsync(&e, dv + 64, 8, cudaMemcpyDeviceToHost, st));
-    sync(ctx);
-    return e;
+    launch_gs_pass(&xp, 1, y, nullptr, 0.0, n, false, env->part.d(), dv + GS_NORM, tk, st, nullptr,
+                   ctx->post.next());
+    return ctx->post.wait(st)[GS_NORM];
 }
 
 // -------------------------------------------------------------------------------------
@@ -2233,7 +2196,8 @@ void replace_bond_noise(tn_env* env, int p, Heff2Plan& P, const double* phi,
     }
     if (prm->normalize && other.lay.size > 0) {
         const double* op = other.buf.d();
-        launch_multi_dot(&op, 1, op, other.lay.size, env->part.d(), env->dots.d() + 64, st);
+        launch_multi_dot(&op, 1, op, other.lay.size, env->part.d(), env->dots.d() + 64,
+                         ctx->gs_ticket.as<unsigned>(), st);
         launch_scale_into(other.buf.d(), other.buf.d(), env->dots.d() + 64, 1.0, other.lay.size, st);
     }
     ctx->timer.add(T_SVD, e1, ctx->timer.mark());
@@ -2929,6 +2893,33 @@ int tn::svd_truncate_dense(tn_ctx* ctx, const double* A, int m, int n, int maxdi
 // EventTimer
 // -------------------------------------------------------------------------------------
 namespace tn {
+HostPost PostBox::next(const double* start) {
+    void* dev = nullptr;
+    TN_CUDA(cudaHostGetDevicePointer(&dev, page, 0));
+    HostPost p;
+    p.values = static_cast<double*>(dev);
+    p.flag = reinterpret_cast<unsigned long long*>(p.values + 128);
+    p.seq = ++seq;
+    p.start = start;
+    return p;
+}
+
+const double* PostBox::wait(cudaStream_t s) {
+    static_assert(GS_VALUES <= 128, "values and flag share the page");
+    const double* values = static_cast<const double*>(page);
+    const auto* flag = reinterpret_cast<const unsigned long long*>(values + 128);
+    auto there = [&] { return __atomic_load_n(flag, __ATOMIC_ACQUIRE) == seq; };
+    for (unsigned spin = 1; !there(); ++spin) {
+        if (spin & 0xfff) continue;
+        // a launch that failed never posts: the stream then reports the error, or ends
+        const cudaError_t e = cudaStreamQuery(s);
+        if (e == cudaErrorNotReady) continue;
+        TN_CUDA(e);
+        TN_REQUIRE(there(), "internal: a kernel ended without posting its results");
+    }
+    return values;
+}
+
 int EventTimer::mark() {
     if (used == pool.size()) {
         cudaEvent_t e;
@@ -2978,6 +2969,10 @@ int tn_ctx_create(int device, tn_ctx** out) {
         c->nsm = pr.multiProcessorCount;
         c->err.alloc(4 * sizeof(int), c->stream);  // [0] error flag, [1] injected wait timeout
         TN_CUDA(cudaMemsetAsync(c->err.p, 0, 4 * sizeof(int), c->stream));
+        c->gs_ticket.alloc(sizeof(unsigned), c->stream);
+        TN_CUDA(cudaMemsetAsync(c->gs_ticket.p, 0, sizeof(unsigned), c->stream));
+        TN_CUDA(cudaHostAlloc(&c->post.page, 4096, cudaHostAllocMapped));
+        std::memset(c->post.page, 0, 4096);
         TN_CUDA(cudaStreamSynchronize(c->stream));
         cudaMemPool_t mp;
         TN_CUDA(cudaDeviceGetDefaultMemPool(&mp, device));

@@ -29,6 +29,22 @@ struct EventTimer {
     ~EventTimer();
 };
 
+// One page of mapped pinned memory through which kernels post small results to the host: the
+// host spins on the sequence number instead of copying and synchronising the stream.  Posts of
+// a context are strictly one after the other (one stream, one caller at a time).
+struct PostBox {
+    void* page = nullptr;
+    unsigned long long seq = 0;
+    PostBox() = default;
+    PostBox(const PostBox&) = delete;
+    PostBox& operator=(const PostBox&) = delete;
+    ~PostBox() {
+        if (page) cudaFreeHost(page);
+    }
+    HostPost next(const double* start = nullptr);    // to be posted by the next launch
+    const double* wait(cudaStream_t s);               // the values, once they are there
+};
+
 struct Scratch;  // fixed-capacity device scratch used by the allocation-free entry points
 
 // work buffers of the multi-SM block SVD (bsvd.cpp), kept by the context between bonds
@@ -98,6 +114,8 @@ struct tn_ctx {
     int prec = TN_PREC_FP64;
     int slices = 5;
     tn::EventTimer timer;
+    tn::PostBox post;
+    tn::DevBuf gs_ticket;  // block counter of the Gram-Schmidt passes (zero between launches)
     tn::DevBuf err;  // device error word of bounded waits (0 = ok)
     int svd_big_n = -1;  // charge blocks with more columns take the multi-SM SVD (-1: tuned)
     tn::SvdTuner svd_tune;
@@ -200,7 +218,7 @@ struct tn_env {
     int lpos = 0, rpos = 0;
     int pos = 0, nsite = 2;
     // work buffers
-    tn::DevBuf t1, t2, kry, part, dots, ticket, svdX, svdW, svdV, svdP, svdS, svdPerm, desc, desc2,
+    tn::DevBuf t1, t2, kry, part, dots, svdX, svdW, svdV, svdP, svdS, svdPerm, desc, desc2,
         vecA, vecB, cx;  // cx: realified complex blocks
     std::unique_ptr<Heff2Plan> hp;
     int hp_pos = -1;

@@ -2,10 +2,12 @@
 //  * grouped block-sparse GEMM (CUDA-core DFMA) -- the FP64 GPU path of every contraction
 //    of the two-site effective Hamiltonian and of the environment updates;
 //  * block linear combination -- the MPO step between the two GEMM stages;
-//  * Krylov vector kernels (multi-dot, multi-axpy, scaling, linear combination) with
+//  * Krylov vector kernels (Gram-Schmidt passes, multi-axpy, scaling, linear combinations) with
 //    warp-shuffle reductions and a deterministic two-stage finalisation.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include "reduce.cuh"
 #include "tn_internal.h"
 
 namespace tn {
@@ -141,7 +143,7 @@ gemm_f64_kernel(const Seg* __restrict__ segs, const Task* __restrict__ tasks,
 
 __global__ void __launch_bounds__(256)
 combine_kernel(const CombOut* __restrict__ outs, const CombTerm* __restrict__ terms,
-               const CombTile* __restrict__ tiles, Bases b) {
+               const CombTile* __restrict__ tiles, const __grid_constant__ Bases b) {
     const CombTile t = tiles[blockIdx.x];
     const CombOut o = outs[t.out];
     const int r = t.r0 + (threadIdx.x & 31);
@@ -181,48 +183,8 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-template <int K>
 __global__ void __launch_bounds__(BLAS_THREADS)
-multi_dot_kernel(VecPtrs V, int kk, const double* __restrict__ w, int64_t n,
-                 double* __restrict__ part) {
-    double acc[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) acc[k] = 0.0;
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const double x = w[i];
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (k < kk) acc[k] = fma(V.p[k][i], x, acc[k]);
-    }
-    __shared__ double red[BLAS_THREADS / 32][K];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const double v = warp_sum(acc[k]);
-        if (lane == 0) red[wid][k] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < kk) {
-        double s = 0.0;
-        for (int j = 0; j < BLAS_THREADS / 32; ++j) s += red[j][threadIdx.x];
-        part[int64_t(threadIdx.x) * gridDim.x + blockIdx.x] = s;
-    }
-}
-
-__global__ void finalize_dot_kernel(const double* __restrict__ part, int nparts, int kk,
-                                    double* __restrict__ out) {
-    // one warp per result, fixed summation order
-    const int k = blockIdx.x;
-    if (k >= kk) return;
-    double s = 0.0;
-    for (int j = threadIdx.x; j < nparts; j += 32) s += part[int64_t(k) * nparts + j];
-    s = warp_sum(s);
-    if (threadIdx.x == 0) out[k] = s;
-}
-
-__global__ void __launch_bounds__(BLAS_THREADS)
-multi_axpy_kernel(double* __restrict__ w, VecPtrs V, int kk, const double* __restrict__ h,
+multi_axpy_kernel(double* __restrict__ w, const __grid_constant__ VecPtrs V, int kk, const double* __restrict__ h,
                   double sign, int64_t n) {
     __shared__ double hs[KMAX];
     if (threadIdx.x < kk) hs[threadIdx.x] = sign * h[threadIdx.x];
@@ -245,65 +207,102 @@ scale_into_kernel(double* __restrict__ dst, const double* __restrict__ src,
         dst[i] = src[i] * s;
 }
 
+// dst_j = sum_k c[j][k] V_k for several outputs in one launch, the coefficients as kernel
+// arguments (a Ritz restart of Lanczos: one upload, launch and host wait per vector before)
+struct LinArgs {
+    double* dst[KMAX];
+    double c[KMAX][KMAX];
+};
 __global__ void __launch_bounds__(BLAS_THREADS)
-lincomb_kernel(double* __restrict__ dst, VecPtrs V, int kk, const double* __restrict__ coef,
-               int64_t n) {
-    __shared__ double cs[KMAX];
-    if (threadIdx.x < kk) cs[threadIdx.x] = coef[threadIdx.x];
-    __syncthreads();
+lincomb_multi_kernel(const __grid_constant__ LinArgs a, const __grid_constant__ VecPtrs V, int nd,
+                     int kk, int64_t n) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        double x = 0.0;
-        for (int k = 0; k < kk; ++k) x = fma(cs[k], V.p[k][i], x);
-        dst[i] = x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
+        for (int j = 0; j < nd; ++j) {
+            double x = 0.0;
+            for (int k = 0; k < kk; ++k) x = fma(a.c[j][k], V.p[k][i], x);
+            a.dst[j][i] = x;
+        }
+}
+
+// dst = sum_k (re_k + i im_k) V_k on planar complex vectors of nc values per plane, real c:
+// the products of the imaginary parts enter as dst_re -= sum im V_im, dst_im += sum im V_re
+struct CLinArgs {
+    double re[KMAX], im[KMAX];
+};
+__global__ void __launch_bounds__(BLAS_THREADS)
+lincomb_complex_kernel(double* __restrict__ dst, const __grid_constant__ CLinArgs a,
+                       const __grid_constant__ VecPtrs V, int kk, int64_t nc) {
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nc; i += stride) {
+        double xr = 0.0, xi = 0.0, wr = 0.0, wi = 0.0;
+        for (int k = 0; k < kk; ++k) {
+            const double vr = V.p[k][i], vi = V.p[k][i + nc];
+            xr = fma(a.re[k], vr, xr);
+            xi = fma(a.re[k], vi, xi);
+            wr = fma(a.im[k], vr, wr);
+            wi = fma(a.im[k], vi, wi);
+        }
+        dst[i] = xr - wi;
+        dst[i + nc] = xi + wr;
     }
 }
 
-// One fused Gram-Schmidt pass over a Krylov residual w:
+// results for the host: `values` in mapped pinned memory, then the sequence number
+__device__ __forceinline__ void host_post(const HostPost& p) {
+    __threadfence_system();
+    if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned long long*>(p.flag) = p.seq;
+}
+
+// One Gram-Schmidt pass over a Krylov residual w:
 //   (optional)  w += sign * sum_k hin[k] V_k
-//   (optional)  out[k] = V_k . w   for k < kk          (with the updated w)
-//   (optional)  out[kk or 0] = w . w
-// Partial sums of every block go to `part`; the last block to finish (atomic ticket)
-// adds them in block order, so results are deterministic, and resets the ticket.
-template <int K>
+//   out[k] = V_k . w for k < kk (with the updated w), or with `norm` out[0] = w . w
+// A block sums 256 elements (and those a whole grid of BLAS_PARTS blocks further on) over warps
+// and then over its warps; the last block to finish (atomic ticket) adds the blocks' sums in
+// block order, so results are deterministic and independent of the grid, which covers n only.
+// With a host post the last block also hands over h1 = post_h1[0..kk), hin and its results.
+//
+// Bound by the FP64 pipe and latency at the sizes of small and middle bonds.  Before, 304
+// blocks of any n and plain butterflies took 10.2 (4 vectors) and 13.5 us (8 vectors) a pass.
+template <int C>
 __global__ void __launch_bounds__(BLAS_THREADS)
-gs_pass_kernel(VecPtrs V, int kk, double* __restrict__ w, const double* __restrict__ hin,
-               double sign, int64_t n, int dots, int norm, double* __restrict__ part,
-               double* __restrict__ out, unsigned* __restrict__ ticket) {
+gs_pass_kernel(const __grid_constant__ VecPtrs V, int kk, double* __restrict__ w,
+               const double* __restrict__ hin, double sign, int64_t n, int norm,
+               double* __restrict__ part, double* __restrict__ out,
+               unsigned* __restrict__ ticket, const double* __restrict__ post_h1,
+               HostPost post) {
     __shared__ double hs[KMAX];
-    __shared__ double red[BLAS_THREADS / 32][K + 1];
+    __shared__ double red[BLAS_THREADS / 32][C];
     __shared__ int last;
     if (hin && threadIdx.x < kk) hs[threadIdx.x] = sign * hin[threadIdx.x];
     __syncthreads();
-    double acc[K + 1];
+    double acc[C];
 #pragma unroll
-    for (int k = 0; k <= K; ++k) acc[k] = 0.0;
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+    for (int k = 0; k < C; ++k) acc[k] = 0.0;
+    const int64_t stride = int64_t(BLAS_PARTS) * BLAS_THREADS;
+    for (int64_t i = int64_t(blockIdx.x) * BLAS_THREADS + threadIdx.x; i < n; i += stride) {
         double x = w[i];
         if (hin) {
             for (int k = 0; k < kk; ++k) x = fma(hs[k], V.p[k][i], x);
             w[i] = x;
         }
-        if (dots) {
+        if (norm) {
+            acc[0] = fma(x, x, acc[0]);
+        } else {
 #pragma unroll
-            for (int k = 0; k < K; ++k)
+            for (int k = 0; k < C; ++k)
                 if (k < kk) acc[k] = fma(V.p[k][i], x, acc[k]);
         }
-        if (norm) acc[K] = fma(x, x, acc[K]);
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nres = (dots ? kk : 0) + (norm ? 1 : 0);
-#pragma unroll
-    for (int k = 0; k <= K; ++k) {
-        const double v = warp_sum(acc[k]);
-        if (lane == 0) red[wid][k] = v;
-    }
+    const int nres = norm ? 1 : kk;
+    const double v = warp_sum_multi<C>(acc, lane);
+    if (warp_sum_owner<C>(lane)) red[wid][warp_sum_index<C>(lane)] = v;
     __syncthreads();
     if (threadIdx.x < nres) {
-        const int src = (dots && threadIdx.x < kk) ? threadIdx.x : K;
         double sum = 0.0;
-        for (int j = 0; j < BLAS_THREADS / 32; ++j) sum += red[j][src];
+#pragma unroll
+        for (int j = 0; j < BLAS_THREADS / 32; ++j) sum += red[j][threadIdx.x];
         part[int64_t(threadIdx.x) * gridDim.x + blockIdx.x] = sum;
     }
     __threadfence();
@@ -317,9 +316,128 @@ gs_pass_kernel(VecPtrs V, int kk, double* __restrict__ w, const double* __restri
         for (int bb = lane; bb < (int)gridDim.x; bb += 32)
             sum += reinterpret_cast<volatile double*>(part)[int64_t(j) * gridDim.x + bb];
         sum = warp_sum(sum);
-        if (lane == 0) out[j] = sum;
+        if (lane == 0) {
+            out[j] = sum;
+            if (post.values) post.values[GS_NORM + j] = sum;
+        }
     }
     if (threadIdx.x == 0) *ticket = 0u;
+    if (post.values) {
+        if (threadIdx.x < kk && post_h1) {
+            post.values[threadIdx.x] = post_h1[threadIdx.x];
+            post.values[GS_H2 + threadIdx.x] = hin[threadIdx.x];
+        }
+        if (threadIdx.x == 0 && post.start) post.values[GS_START] = *post.start;
+        __syncthreads();
+        host_post(post);
+    }
+}
+
+// The whole double Gram-Schmidt step of a short residual in one launch:
+//   h1 = V^T w, w -= V h1, h2 = V^T w, w -= V h2, |w|^2, next = w / |w|
+// A cluster of CL CTAs keeps w in registers, each thread one element of up to GS2_PARTS parts of
+// 256 elements; the parts' sums meet through distributed shared memory.  The sums are formed
+// in gs_pass_kernel's order (element, warp, the part's eight warps, parts by lane), so the
+// results are the same bits as its three passes.
+// Three passes and the scaling of the next vector were four launches and at least 34 us for any
+// n; this is one (12-site DMRG run 71 -> 47 ms, 64-site run in split precision 565 -> 440 ms,
+// both with the results posted to the host).  Every CTA sums all parts by itself and FP64 adds
+// are slow, so it is for short vectors (gs2_cluster): from P (2 K + 4) = 256 on (P parts, K
+// vectors) the passes, which spread the parts over all SMs, are as fast.
+constexpr int GS2_PARTS = 4;
+template <int C>
+__global__ void __launch_bounds__(BLAS_THREADS, 1)
+gs2_kernel(const __grid_constant__ VecPtrs V, int kk, double* __restrict__ w,
+           double* __restrict__ next, int n, double* __restrict__ out, HostPost post) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ double red[BLAS_THREADS / 32][C];
+    __shared__ double sums[3][GS2_PARTS][C];  // this CTA's parts, one array per phase
+    __shared__ double hs[C];
+    const int CL = int(cl.num_blocks()), rank = int(cl.block_rank());
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int P = (n + BLAS_THREADS - 1) / BLAS_THREADS;  // part p: CTA p % CL, slot p / CL
+    double x[GS2_PARTS];
+#pragma unroll
+    for (int s = 0; s < GS2_PARTS; ++s) {
+        const int i = (s * CL + rank) * BLAS_THREADS + int(threadIdx.x);
+        x[s] = i < n ? w[i] : 0.0;
+    }
+    // sums over the parts of phase f for every result, into hs (all CTAs alike)
+    auto finish = [&](int f, int nres) {
+        cl.sync();
+        for (int j = wid; j < nres; j += BLAS_THREADS / 32) {
+            double s = 0.0;
+            if (lane < P) s = cl.map_shared_rank(&sums[f][lane / CL][j], lane % CL)[0];
+            s = warp_sum(s);
+            if (lane == 0) hs[j] = s;
+        }
+        __syncthreads();
+    };
+    auto part_sum = [&](int f, int s, double v, int nres, bool owner, int idx) {
+        if (owner) red[wid][idx] = v;
+        __syncthreads();
+        if (threadIdx.x < nres) {
+            double sum = 0.0;
+#pragma unroll
+            for (int j = 0; j < BLAS_THREADS / 32; ++j) sum += red[j][threadIdx.x];
+            sums[f][s][threadIdx.x] = sum;
+        }
+        __syncthreads();
+    };
+#pragma unroll 1
+    for (int f = 0; f < 2; ++f) {
+#pragma unroll
+        for (int s = 0; s < GS2_PARTS; ++s) {
+            if (s * CL + rank >= P) break;
+            const int i = (s * CL + rank) * BLAS_THREADS + int(threadIdx.x);
+            double acc[C];
+#pragma unroll
+            for (int k = 0; k < C; ++k) acc[k] = (k < kk && i < n) ? fma(V.p[k][i], x[s], 0.0) : 0.0;
+            const double v = warp_sum_multi<C>(acc, lane);
+            part_sum(f, s, v, kk, warp_sum_owner<C>(lane), warp_sum_index<C>(lane));
+        }
+        finish(f, kk);
+        if (rank == 0 && threadIdx.x < kk) {
+            const double h = hs[threadIdx.x];
+            out[f * GS_H2 + threadIdx.x] = h;
+            post.values[f * GS_H2 + threadIdx.x] = h;
+        }
+#pragma unroll
+        for (int s = 0; s < GS2_PARTS; ++s) {
+            const int i = (s * CL + rank) * BLAS_THREADS + int(threadIdx.x);
+            if (i < n)
+                for (int k = 0; k < kk; ++k) x[s] = fma(-hs[k], V.p[k][i], x[s]);
+        }
+        __syncthreads();  // hs is read until here
+    }
+#pragma unroll
+    for (int s = 0; s < GS2_PARTS; ++s) {
+        if (s * CL + rank >= P) break;
+        const double v = warp_sum(fma(x[s], x[s], 0.0));
+        part_sum(2, s, v, 1, lane == 0, 0);
+    }
+    finish(2, 1);
+    const double nrm = hs[0];
+    const double scale = 1.0 / sqrt(nrm);
+#pragma unroll
+    for (int s = 0; s < GS2_PARTS; ++s) {
+        const int i = (s * CL + rank) * BLAS_THREADS + int(threadIdx.x);
+        if (i < n) {
+            w[i] = x[s];
+            if (next) next[i] = x[s] * scale;
+        }
+    }
+    if (rank == 0) {
+        if (threadIdx.x == 0) {
+            out[GS_NORM] = nrm;
+            post.values[GS_NORM] = nrm;
+            if (post.start) post.values[GS_START] = *post.start;
+        }
+        __syncthreads();
+        host_post(post);
+    }
+    cl.sync();  // the other CTAs read this one's sums until here
 }
 
 __global__ void __launch_bounds__(BLAS_THREADS)
@@ -386,24 +504,9 @@ void launch_block_dots(const BlockDot* d, int n, double* out, cudaStream_t s) {
 }
 
 void launch_multi_dot(const double* const* V, int K, const double* w, int64_t n,
-                      double* part, double* out, cudaStream_t s) {
+                      double* part, double* out, unsigned* ticket, cudaStream_t s) {
     if (K <= 0) return;
-    VecPtrs P = make_ptrs(V, K);
-    const int g = BLAS_PARTS;  // fixed part count: deterministic, finalize reads g parts
-    if (K <= 4)
-        multi_dot_kernel<4><<<g, BLAS_THREADS, 0, s>>>(P, K, w, n, part);
-    else if (K <= 8)
-        multi_dot_kernel<8><<<g, BLAS_THREADS, 0, s>>>(P, K, w, n, part);
-    else if (K <= 16)
-        multi_dot_kernel<16><<<g, BLAS_THREADS, 0, s>>>(P, K, w, n, part);
-    else
-        multi_dot_kernel<32><<<g, BLAS_THREADS, 0, s>>>(P, K, w, n, part);
-    TN_CUDA(cudaGetLastError());
-    count_launch();
-    finalize_dot_kernel<<<K, 32, 0, s>>>(part, g, K, out);
-    TN_CUDA(cudaGetLastError());
-    count_launch();
-    count_krylov_bytes(int64_t(K + 1) * n * 8);
+    launch_gs_pass(V, K, const_cast<double*>(w), nullptr, 0.0, n, false, part, out, ticket, s);
 }
 
 void launch_multi_axpy(double* w, const double* const* V, int K, const double* h, double sign,
@@ -416,22 +519,61 @@ void launch_multi_axpy(double* w, const double* const* V, int K, const double* h
 }
 
 void launch_gs_pass(const double* const* V, int K, double* w, const double* hin, double sign,
-                    int64_t n, bool dots, bool norm, double* part, double* out, unsigned* ticket,
-                    cudaStream_t s) {
+                    int64_t n, bool norm, double* part, double* out, unsigned* ticket,
+                    cudaStream_t s, const double* post_h1, const HostPost& post) {
     VecPtrs P = K > 0 ? make_ptrs(V, K) : VecPtrs{};
-    const int g = BLAS_PARTS;
-    const int d = dots ? 1 : 0, nm = norm ? 1 : 0;
-    if (K <= 4)
-        gs_pass_kernel<4><<<g, BLAS_THREADS, 0, s>>>(P, K, w, hin, sign, n, d, nm, part, out, ticket);
-    else if (K <= 8)
-        gs_pass_kernel<8><<<g, BLAS_THREADS, 0, s>>>(P, K, w, hin, sign, n, d, nm, part, out, ticket);
-    else if (K <= 16)
-        gs_pass_kernel<16><<<g, BLAS_THREADS, 0, s>>>(P, K, w, hin, sign, n, d, nm, part, out, ticket);
-    else
-        gs_pass_kernel<32><<<g, BLAS_THREADS, 0, s>>>(P, K, w, hin, sign, n, d, nm, part, out, ticket);
+    const int g = grid_for(n);
+    const int nm = norm ? 1 : 0, nres = norm ? 1 : K;
+    auto* kernel = nres <= 1    ? gs_pass_kernel<1>
+                   : nres <= 2  ? gs_pass_kernel<2>
+                   : nres <= 4  ? gs_pass_kernel<4>
+                   : nres <= 8  ? gs_pass_kernel<8>
+                   : nres <= 16 ? gs_pass_kernel<16>
+                                : gs_pass_kernel<32>;
+    kernel<<<g, BLAS_THREADS, 0, s>>>(P, K, w, hin, sign, n, nm, part, out, ticket, post_h1, post);
     TN_CUDA(cudaGetLastError());
     count_launch();
-    count_krylov_bytes(int64_t(1 + ((hin || dots) ? K : 0) + (hin ? 1 : 0)) * n * 8);
+    count_krylov_bytes(int64_t(1 + ((hin || !norm) ? K : 0) + (hin ? 1 : 0)) * n * 8);
+}
+
+// CTAs of gs2_kernel's cluster for n elements and K vectors, 0: too long for it
+static int gs2_cluster(int64_t n, int K) {
+    const int64_t P = (n + BLAS_THREADS - 1) / BLAS_THREADS;
+    if (P < 1 || P > 8 * GS2_PARTS || P * (2 * K + 4) > 256) return 0;
+    int c = 1;
+    while (c < 8 && c < P) c *= 2;
+    return c;
+}
+
+void launch_gs2(const double* const* V, int K, double* w, double* next, int64_t n, double* part,
+                double* out, unsigned* ticket, const HostPost& post, cudaStream_t s) {
+    const int c = gs2_cluster(n, K);
+    if (c == 0) {
+        launch_gs_pass(V, K, w, nullptr, 0.0, n, false, part, out, ticket, s);
+        launch_gs_pass(V, K, w, out, -1.0, n, false, part, out + GS_H2, ticket, s);
+        launch_gs_pass(V, K, w, out + GS_H2, -1.0, n, true, part, out + GS_NORM, ticket, s, out, post);
+        if (next) launch_scale_into(next, w, out + GS_NORM, 1.0, n, s);
+        return;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(c));
+    cfg.blockDim = dim3(BLAS_THREADS);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = unsigned(c);
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    auto* kernel = K <= 1    ? gs2_kernel<1>
+                   : K <= 2  ? gs2_kernel<2>
+                   : K <= 4  ? gs2_kernel<4>
+                   : K <= 8  ? gs2_kernel<8>
+                   : K <= 16 ? gs2_kernel<16>
+                             : gs2_kernel<32>;
+    TN_CUDA(cudaLaunchKernelEx(&cfg, kernel, make_ptrs(V, K), K, w, next, int(n), out, post));
+    count_launch();
+    count_krylov_bytes(int64_t(2 * K + 2 + (next ? 1 : 0)) * n * 8);
 }
 
 void launch_scale_into(double* dst, const double* src, const double* denom_sq,
@@ -443,13 +585,34 @@ void launch_scale_into(double* dst, const double* src, const double* denom_sq,
     count_krylov_bytes(2 * n * 8);
 }
 
-void launch_lincomb(double* dst, const double* const* V, int K, const double* coef, int64_t n,
-                    cudaStream_t s) {
-    if (n <= 0) return;
-    lincomb_kernel<<<grid_for(n), BLAS_THREADS, 0, s>>>(dst, make_ptrs(V, K), K, coef, n);
+void launch_lincomb(double* const* dst, int nd, const double* const* V, int K,
+                    const double* coef, int64_t n, cudaStream_t s) {
+    if (n <= 0 || nd <= 0) return;
+    TN_REQUIRE(nd <= KMAX, "too many linear combinations for one kernel");
+    LinArgs a;
+    for (int j = 0; j < nd; ++j) {
+        a.dst[j] = dst[j];
+        for (int k = 0; k < K; ++k) a.c[j][k] = coef[j * K + k];
+    }
+    lincomb_multi_kernel<<<grid_for(n), BLAS_THREADS, 0, s>>>(a, make_ptrs(V, K), nd, K, n);
     TN_CUDA(cudaGetLastError());
     count_launch();
-    count_krylov_bytes(int64_t(K + 1) * n * 8);
+    count_krylov_bytes(int64_t(K + 1) * nd * n * 8);
+}
+
+void launch_lincomb_complex(double* dst, const double* const* V, int K, const double* re,
+                            const double* im, int64_t nc, cudaStream_t s) {
+    if (nc <= 0) return;
+    CLinArgs a;
+    VecPtrs P = make_ptrs(V, K);
+    for (int k = 0; k < K; ++k) {
+        a.re[k] = re[k];
+        a.im[k] = im[k];
+    }
+    lincomb_complex_kernel<<<grid_for(nc), BLAS_THREADS, 0, s>>>(dst, a, P, K, nc);
+    TN_CUDA(cudaGetLastError());
+    count_launch();
+    count_krylov_bytes(int64_t(K + 1) * 2 * nc * 8);
 }
 
 }  // namespace tn

@@ -366,7 +366,8 @@ void proj_apply(tn_env* env, const double* x, double* y, int64_t n) {
     std::vector<const double*> m(K);
     for (int k = 0; k < K; ++k) m[k] = env->projm.d() + int64_t(k) * n;
     env->projc.alloc(64 * 8, st);
-    launch_multi_dot(m.data(), K, x, n, env->part.d(), env->projc.d(), st);
+    launch_multi_dot(m.data(), K, x, n, env->part.d(), env->projc.d(),
+                     env->ctx->gs_ticket.as<unsigned>(), st);
     launch_multi_axpy(y, m.data(), K, env->projc.d(), env->proj_weight, n, st);
 }
 

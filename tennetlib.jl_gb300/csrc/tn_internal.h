@@ -259,18 +259,37 @@ void launch_combine(const CombPlan& p, const Bases& b, cudaStream_t s);
 // finalized results to `out` (K doubles), all on the device.
 int blas_nparts();
 void launch_multi_dot(const double* const* V, int K, const double* w, int64_t n,
-                      double* part, double* out, cudaStream_t s);
+                      double* part, double* out, unsigned* ticket, cudaStream_t s);
 void launch_multi_axpy(double* w, const double* const* V, int K, const double* h,
                        double sign, int64_t n, cudaStream_t s);
-// Fused Gram-Schmidt pass (see kernels_f64.cu): optional w += sign * V hin, optional dots
-// V^T w into out[0..K), optional |w|^2 into out[K or 0]; one launch, deterministic.
+// Results posted by a kernel to mapped pinned host memory: values, then *flag = seq (values
+// null: nothing is posted).  start: one more device value to post.
+struct HostPost {
+    double* values = nullptr;
+    unsigned long long* flag = nullptr;
+    unsigned long long seq = 0;
+    const double* start = nullptr;
+};
+// offsets in the device results and the posted values of a Gram-Schmidt step
+constexpr int GS_H2 = 32, GS_NORM = 64, GS_START = 65, GS_VALUES = 66;
+// One Gram-Schmidt pass (see kernels_f64.cu): optional w += sign * V hin, then V^T w into
+// out[0..K), or with norm |w|^2 into out[0]; one launch, deterministic.
 void launch_gs_pass(const double* const* V, int K, double* w, const double* hin, double sign,
-                    int64_t n, bool dots, bool norm, double* part, double* out, unsigned* ticket,
-                    cudaStream_t s);
+                    int64_t n, bool norm, double* part, double* out, unsigned* ticket,
+                    cudaStream_t s, const double* post_h1 = nullptr, const HostPost& post = {});
+// Double Gram-Schmidt step of the residual w against V: both coefficient vectors (out, out +
+// GS_H2) and |w|^2 (out + GS_NORM) on the device and posted to the host; next (or null) gets
+// w / |w|.
+void launch_gs2(const double* const* V, int K, double* w, double* next, int64_t n, double* part,
+                double* out, unsigned* ticket, const HostPost& post, cudaStream_t s);
 void launch_scale_into(double* dst, const double* src, const double* denom_sq_or_null,
                        double host_scale, int64_t n, cudaStream_t s);
-void launch_lincomb(double* dst, const double* const* V, int K, const double* coef,
-                    int64_t n, cudaStream_t s);
+// dst[j] = sum_k coef[j * K + k] V_k, coefficients on the host
+void launch_lincomb(double* const* dst, int nd, const double* const* V, int K,
+                    const double* coef, int64_t n, cudaStream_t s);
+// dst = sum_k (re_k + i im_k) V_k on planar complex vectors (nc values per plane)
+void launch_lincomb_complex(double* dst, const double* const* V, int K, const double* re,
+                            const double* im, int64_t nc, cudaStream_t s);
 
 // sum of x (.) y over one rows x cols block pair (x, y column-major with their leading
 // dimensions), one result per pair, deterministic

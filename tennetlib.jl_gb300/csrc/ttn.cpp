@@ -991,7 +991,7 @@ void proj_apply(TtnGroup& G, int node) {
         std::vector<const double*> m(K);
         for (int k = 0; k < K; ++k) m[k] = e->proj_m.d() + int64_t(k) * S;
         launch_multi_dot(m.data(), K, wptr(G, e, e->w_x), n, e->proj_part.d(), e->proj_c.d(),
-                         G.ctx->stream);
+                         G.ctx->gs_ticket.as<unsigned>(), G.ctx->stream);
         launch_multi_axpy(wptr(G, e, e->w_y), m.data(), K, e->proj_c.d(), e->proj_weight, n,
                           G.ctx->stream);
     }
