@@ -258,6 +258,8 @@ std::unique_ptr<SplitPlan> make_split(const GemmPlan& g, int slices, bool a_stat
         stsk.ea_off = anew ? int32_t(eao) : int32_t(ait->second.second);
         stsk.eb_off = bnew ? int32_t(ebo) : int32_t(bit->second.second);
         stsk.accum = t.accum;
+        for (int j = 0; j < std::min(nkt, SPLIT_KMASK); ++j)
+            stsk.kmask |= uint64_t((kts[size_t(j)].kv + 15) / 16 - 1) << (2 * j);
         sp->tasks.push_back(stsk);
         const int akt0 = (int)sp->aks.size(), bkt0 = (int)sp->bks.size();
         for (const auto& k : kts) {

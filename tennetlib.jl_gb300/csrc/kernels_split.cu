@@ -19,6 +19,11 @@
 //    Every chunk of two k tiles the epilogue drains the accumulators (double-buffered in
 //    TMEM) into (hi, lo) FP32 pairs with error-free additions; at the end of the tile the
 //    pair is rescaled by 2^(E_row + E_col - 16) in FP64 and stored.
+// Small blocks (a chi = 50 bond has blocks of 15 to 30 rows) use a corner of their 128 x 64 tile
+// and 64-deep k tiles: only the 8-row atoms that hold rows are copied, only the 16-deep steps
+// with valid k and the columns of the block are multiplied, only its columns and row quadrants
+// are drained and converted, each as before to the bit (22.9 -> 15.6 us per launch there, with
+// the packs 69 -> 44 us per H_eff product; 64-site DMRG run 440 -> 360 ms).
 // Every mbarrier wait is bounded (about one second); a wait that gives up sets the error
 // word, and all roles then drain with bounded waits, free TMEM and return.
 #include <cuda_bf16.h>
@@ -136,17 +141,23 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-    uint32_t r[16];
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
         "%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-          "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
+          "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]),
+          "=f"(v[14]), "=f"(v[15])
         : "r"(taddr));
+}
+
+// waits for the loads above; the values pass through it, so that none is read before
+__device__ __forceinline__ void tmem_wait(float (&v)[NACC][16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+    for (int l = 0; l < NACC; ++l)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) asm volatile("" : "+f"(v[l][c]));
 }
 
 // error-free addition of a into (hi, lo) (Knuth's TwoSum, lo collects the rounding errors)
@@ -162,106 +173,137 @@ __device__ __forceinline__ double pow2(int e) {
     return __longlong_as_double(static_cast<long long>(1023 + e) << 52);
 }
 
+// double(x), exactly, on the integer pipe for zeros and normal numbers (a conversion holds the
+// FP64 pipe as long as an add does)
+__device__ __forceinline__ double widen(float x) {
+    const unsigned u = __float_as_uint(x), a = u & 0x7fffffffu;
+    if (a - 0x00800000u >= 0x7f000000u && a != 0u) return double(x);  // subnormal, inf, NaN
+    const unsigned hi = a ? (a >> 3) + 0x38000000u : 0u;
+    return __hiloint2double(int(hi | (u & 0x80000000u)), int(u << 29));
+}
+
+// v * 2^e, exactly the product: on the exponent field while both v and the result are normal
+__device__ __forceinline__ double scale2(double v, int e) {
+    const int hi = __double2hiint(v), ex = (hi >> 20) & 0x7ff;
+    if (ex == 0 || ex == 0x7ff || unsigned(ex + e - 1) >= 2046u) return v * pow2(e);
+    return __hiloint2double(hi + (e << 20), __double2loint(v));
+}
+
 // ------------------------------------------------------------------------------------
-// pack kernel: a row tile (128 rows for A, 64 for B) is shared by tile_rows / PACK_ROWS CTAs
-// (gridDim.y), each packing all k tiles of its PACK_ROWS rows: the row maxima stay within a
-// CTA, and small operands still spread over many SMs
+// pack kernels.  Only what the MMA kernel copies and multiplies is written: rows up to the
+// next multiple of 8 (one swizzle atom), and of a k tile the 16-deep MMA steps that hold valid
+// k (split_ksteps; a charge block of 14 x 14 fills 16 rows and one step of four, a sixteenth of
+// its A tile).
 // ------------------------------------------------------------------------------------
 constexpr int PACK_THREADS = 256;
-constexpr int PACK_ROWS = 32;
+constexpr int PACK_ROWS = 8;
 
-// Work item of the pack kernel: row r of the tile and one 8-wide chunk (16 bytes of bf16)
-// of one k tile; consecutive threads take consecutive rows so that the loads of a column-
-// major operand coalesce, and each thread keeps 8 independent loads in flight.
+// 8-wide chunks of k tile t that are packed
+__device__ __forceinline__ int pack_chunks(int t, int kvalid) {
+    return t < SPLIT_KMASK ? 2 * ((kvalid + 15) / 16) : BKT / 8;
+}
+
+// Eight elements of row r (chunk ch of a k tile at tile0): balanced base-256 digits.
+// x * 2^(8s - E) = sig * 2^(ex - 1075 + 8s - E), sig the 53-bit significand: the rounded
+// integer is sig shifted right by sh = 1075 + E - 8s - ex (round half away from zero), integer
+// pipe only.  mxb is the row's largest |x| as a bit pattern, 0 for an empty row.
+__device__ __forceinline__ void pack_digits(const long long (&v)[8], unsigned long long mxb,
+                                            int r, int ch, uint8_t* tile0, int tile_bytes,
+                                            int slices) {
+    const int E = mxb ? int((mxb >> 52) & 0x7ff) - 1022 : 0;
+    const int base_sh = 1075 + E - 8 * slices;
+    __nv_bfloat16 dig[7][8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        long long X = 0;
+        const int ex = int((v[q] >> 52) & 0x7ff);
+        if (mxb && ex) {  // subnormals are far below the row scale: they round to 0
+            const long long m = (v[q] & 0xfffffffffffffLL) | (1LL << 52);
+            const int sh = base_sh - ex;
+            long long a = 0;
+            if (sh <= 0) a = m << (-sh);
+            else if (sh < 63) a = (m + (1LL << (sh - 1))) >> sh;
+            X = v[q] < 0 ? -a : a;
+        }
+        // compile-time slice indices keep dig[][] in registers
+#pragma unroll
+        for (int i = 6; i >= 1; --i) {
+            if (i >= slices) continue;
+            int d = int(X & 255);
+            if (d > 128) d -= 256;
+            X = (X - d) >> 8;
+            dig[i][q] = __float2bfloat16_rn(ldexpf(float(d), -8 * i));
+        }
+        dig[0][q] = __float2bfloat16_rn(float(X));
+    }
+    // swizzled position of (row r, chunk ch): 8-row atoms of 1024 bytes
+    const int off = (r >> 3) * 1024 + (r & 7) * 128 + ((ch ^ (r & 7)) << 4);
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        if (i >= slices) continue;
+        uint4 w;
+        __builtin_memcpy(&w, dig[i], 16);
+        *reinterpret_cast<uint4*>(tile0 + int64_t(i) * tile_bytes + off) = w;
+    }
+}
+
+// the chunk's elements (zeros beyond the rows and valid k) and their largest |x|
+__device__ __forceinline__ unsigned long long pack_load(long long (&v)[8], const KTileSrc& ks,
+                                                        const Bases& b, int row, bool live, int ch) {
+    const long long* x = reinterpret_cast<const long long*>(b.p[ks.buf] + ks.off) +
+                         int64_t(row) * ks.sr;
+    unsigned long long mx = 0ull;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int k = ch * 8 + q;
+        v[q] = live && k < ks.kvalid ? x[int64_t(k) * ks.sk] : 0ll;
+        const unsigned long long a = (unsigned long long)v[q] & 0x7fffffffffffffffull;
+        mx = a > mx ? a : mx;
+    }
+    return mx;
+}
+
+// A row tile is shared by CTAs of PACK_ROWS rows (gridDim.y), each packing all k tiles of its
+// rows: the row maxima stay within a CTA.  Work item: one row and one 8-wide chunk (16 bytes of
+// bf16) of one k tile; consecutive threads take consecutive rows so that the loads of a
+// column-major operand come in 64-byte pieces, and each thread keeps 8 loads in flight.  Bound
+// by load latency: 8 rows of up to four k tiles are one item per thread, whose elements stay in
+// registers between the maximum and the digits.  With 32 rows per CTA and whole tiles written
+// it took 12.4 us per launch on the blocks of a chi = 50 bond, now 6.2 us.
 __global__ void __launch_bounds__(PACK_THREADS)
-split_pack_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict__ ksrc, Bases b,
-                  uint8_t* __restrict__ out, int* __restrict__ expo, int slices, int tile_rows) {
+split_pack_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict__ ksrc,
+                  const __grid_constant__ Bases b, uint8_t* __restrict__ out,
+                  int* __restrict__ expo, int slices, int tile_rows) {
     __shared__ unsigned long long rowmax[PACK_ROWS];
     const PackJob jb = jobs[blockIdx.x];
     const int r0 = blockIdx.y * PACK_ROWS;
-    const int nr = (tile_rows - r0) < PACK_ROWS ? (tile_rows - r0) : PACK_ROWS;
-    if (nr <= 0) return;
+    if (r0 >= jb.rows) return;
     const int tile_bytes = tile_rows * BKT * 2;
-    const int per_tile = nr * 8;                    // (row, chunk) items per k tile
-    const int nitems = per_tile * jb.nkt;
-    for (int r = threadIdx.x; r < nr; r += blockDim.x) rowmax[r] = 0ull;
+    constexpr int PER_TILE = PACK_ROWS * 8;         // (row, chunk) items per k tile
+    const int nitems = PER_TILE * jb.nkt;
+    if (threadIdx.x < PACK_ROWS) rowmax[threadIdx.x] = 0ull;
     __syncthreads();
-    // pass 1: row maxima of |x| as IEEE bit patterns (integer compare, no FP64 pipe)
-    for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-        const int t = it / per_tile, rem = it % per_tile;
-        const int rl = rem % nr, ch = rem / nr, r = r0 + rl;
-        if (r >= jb.rows) continue;
-        const KTileSrc ks = ksrc[jb.kt0 + t];
-        const long long* x = reinterpret_cast<const long long*>(b.p[ks.buf] + ks.off) +
-                             int64_t(jb.row0 + r) * ks.sr;
-        unsigned long long mx = 0ull;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int k = ch * 8 + q;
-            if (k < ks.kvalid) {
-                const unsigned long long v = (unsigned long long)(x[int64_t(k) * ks.sk]) & 0x7fffffffffffffffull;
-                mx = v > mx ? v : mx;
-            }
-        }
+    const int rl = threadIdx.x % PACK_ROWS, r = r0 + rl;
+    const bool live = r < jb.rows;
+    long long v[8];
+    // row maxima of |x| as IEEE bit patterns (integer compare, no FP64 pipe)
+    for (int it = threadIdx.x; it < nitems; it += PACK_THREADS) {
+        const KTileSrc ks = ksrc[jb.kt0 + it / PER_TILE];
+        const unsigned long long mx =
+            pack_load(v, ks, b, jb.row0 + r, live, (it % PER_TILE) / PACK_ROWS);
         if (mx) atomicMax(&rowmax[rl], mx);
     }
     __syncthreads();
-    for (int rl = threadIdx.x; rl < nr && r0 + rl < jb.rows; rl += blockDim.x) {
-        const unsigned long long m = rowmax[rl];
-        expo[jb.eoff + r0 + rl] = m ? int((m >> 52) & 0x7ff) - 1022 : 0;
-    }
-    // pass 2: balanced base-256 digits.  x * 2^(8s - E) = sig * 2^(ex - 1075 + 8s - E), sig
-    // the 53-bit significand: the rounded integer is sig shifted right by
-    // sh = 1075 + E - 8s - ex (round half away from zero), integer pipe only.
-    for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-        const int t = it / per_tile, rem = it % per_tile;
-        const int rl = rem % nr, ch = rem / nr, r = r0 + rl;
+    const unsigned long long mxb = rowmax[rl];
+    if (threadIdx.x < PACK_ROWS && live)
+        expo[jb.eoff + r] = mxb ? int((mxb >> 52) & 0x7ff) - 1022 : 0;
+    for (int it = threadIdx.x; it < nitems; it += PACK_THREADS) {
+        const int t = it / PER_TILE, ch = (it % PER_TILE) / PACK_ROWS;
         const KTileSrc ks = ksrc[jb.kt0 + t];
-        const bool live = r < jb.rows && ks.kvalid > 0;
-        const unsigned long long mxb = live ? rowmax[rl] : 0ull;
-        const int E = mxb ? int((mxb >> 52) & 0x7ff) - 1022 : 0;
-        const int base_sh = 1075 + E - 8 * slices;
-        const long long* x = live ? reinterpret_cast<const long long*>(b.p[ks.buf] + ks.off) +
-                                        int64_t(jb.row0 + r) * ks.sr
-                                  : nullptr;
-        __nv_bfloat16 dig[7][8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int k = ch * 8 + q;
-            long long X = 0;
-            if (mxb && k < ks.kvalid) {
-                const long long v = x[int64_t(k) * ks.sk];
-                const int ex = int((v >> 52) & 0x7ff);
-                if (ex) {  // subnormals are far below the row scale: they round to 0
-                    const long long m = (v & 0xfffffffffffffLL) | (1LL << 52);
-                    const int sh = base_sh - ex;
-                    long long a = 0;
-                    if (sh <= 0) a = m << (-sh);
-                    else if (sh < 63) a = (m + (1LL << (sh - 1))) >> sh;
-                    X = v < 0 ? -a : a;
-                }
-            }
-            // compile-time slice indices keep dig[][] in registers
-#pragma unroll
-            for (int i = 6; i >= 1; --i) {
-                if (i >= slices) continue;
-                int d = int(X & 255);
-                if (d > 128) d -= 256;
-                X = (X - d) >> 8;
-                dig[i][q] = __float2bfloat16_rn(ldexpf(float(d), -8 * i));
-            }
-            dig[0][q] = __float2bfloat16_rn(float(X));
-        }
-        // swizzled position of (row r, chunk ch): 8-row atoms of 1024 bytes
-        uint8_t* tile0 = out + jb.out_off + int64_t(t) * slices * tile_bytes;
-        const int off = (r >> 3) * 1024 + (r & 7) * 128 + ((ch ^ (r & 7)) << 4);
-#pragma unroll
-        for (int i = 0; i < 7; ++i) {
-            if (i >= slices) continue;
-            uint4 v;
-            __builtin_memcpy(&v, dig[i], 16);
-            *reinterpret_cast<uint4*>(tile0 + int64_t(i) * tile_bytes + off) = v;
-        }
+        if (ch >= pack_chunks(t, ks.kvalid)) continue;
+        if (nitems > PACK_THREADS) pack_load(v, ks, b, jb.row0 + r, live, ch);
+        pack_digits(v, mxb, r, ch, out + jb.out_off + int64_t(t) * slices * tile_bytes, tile_bytes,
+                    slices);
     }
 }
 
@@ -271,33 +313,24 @@ split_pack_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict__
 // pass 2 (split_pack_part_kernel) writes the digits of its k tiles with the exponents taken
 // from gmax.  Same digits as split_pack_kernel, many more CTAs.
 __global__ void __launch_bounds__(PACK_THREADS)
-split_rowmax_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict__ ksrc, Bases b,
-                    unsigned long long* __restrict__ gmax, int tile_rows, int kper) {
+split_rowmax_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict__ ksrc,
+                    const __grid_constant__ Bases b, unsigned long long* __restrict__ gmax,
+                    int kper) {
     __shared__ unsigned long long rowmax[BM];
     const PackJob jb = jobs[blockIdx.x];
     const int t0 = blockIdx.y * kper;
     if (t0 >= jb.nkt) return;
     const int t1 = (t0 + kper) < jb.nkt ? (t0 + kper) : jb.nkt;
-    const int per_tile = tile_rows * 8;
+    const int per_tile = jb.rows * 8;
     const int nitems = per_tile * (t1 - t0);
-    for (int r = threadIdx.x; r < tile_rows; r += blockDim.x) rowmax[r] = 0ull;
+    for (int r = threadIdx.x; r < jb.rows; r += blockDim.x) rowmax[r] = 0ull;
     __syncthreads();
     for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
         const int t = t0 + it / per_tile, rem = it % per_tile;
-        const int r = rem % tile_rows, ch = rem / tile_rows;
-        if (r >= jb.rows) continue;
+        const int r = rem % jb.rows, ch = rem / jb.rows;
         const KTileSrc ks = ksrc[jb.kt0 + t];
-        const long long* x = reinterpret_cast<const long long*>(b.p[ks.buf] + ks.off) +
-                             int64_t(jb.row0 + r) * ks.sr;
-        unsigned long long mx = 0ull;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int k = ch * 8 + q;
-            if (k < ks.kvalid) {
-                const unsigned long long v = (unsigned long long)(x[int64_t(k) * ks.sk]) & 0x7fffffffffffffffull;
-                mx = v > mx ? v : mx;
-            }
-        }
+        long long v[8];
+        const unsigned long long mx = pack_load(v, ks, b, jb.row0 + r, true, ch);
         if (mx) atomicMax(&rowmax[r], mx);
     }
     __syncthreads();
@@ -306,16 +339,17 @@ split_rowmax_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict
 }
 
 __global__ void __launch_bounds__(PACK_THREADS)
-split_pack_part_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict__ ksrc, Bases b,
-                       uint8_t* __restrict__ out, int* __restrict__ expo,
-                       const unsigned long long* __restrict__ gmax, int slices, int tile_rows,
-                       int kper) {
+split_pack_part_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict__ ksrc,
+                       const __grid_constant__ Bases b, uint8_t* __restrict__ out,
+                       int* __restrict__ expo, const unsigned long long* __restrict__ gmax,
+                       int slices, int tile_rows, int kper) {
     const PackJob jb = jobs[blockIdx.x];
     const int t0 = blockIdx.y * kper;
     if (t0 >= jb.nkt) return;
     const int t1 = (t0 + kper) < jb.nkt ? (t0 + kper) : jb.nkt;
     const int tile_bytes = tile_rows * BKT * 2;
-    const int per_tile = tile_rows * 8;
+    const int rows8 = (jb.rows + 7) & ~7;
+    const int per_tile = rows8 * 8;
     const int nitems = per_tile * (t1 - t0);
     if (blockIdx.y == 0)
         for (int r = threadIdx.x; r < jb.rows; r += blockDim.x) {
@@ -324,52 +358,15 @@ split_pack_part_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restr
         }
     for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
         const int t = t0 + it / per_tile, rem = it % per_tile;
-        const int r = rem % tile_rows, ch = rem / tile_rows;
+        const int r = rem % rows8, ch = rem / rows8;
         const KTileSrc ks = ksrc[jb.kt0 + t];
-        const bool live = r < jb.rows && ks.kvalid > 0;
+        if (ch >= pack_chunks(t, ks.kvalid)) continue;
+        const bool live = r < jb.rows;
         const unsigned long long mxb = live ? gmax[jb.eoff + r] : 0ull;
-        const int E = mxb ? int((mxb >> 52) & 0x7ff) - 1022 : 0;
-        const int base_sh = 1075 + E - 8 * slices;
-        const long long* x = live ? reinterpret_cast<const long long*>(b.p[ks.buf] + ks.off) +
-                                        int64_t(jb.row0 + r) * ks.sr
-                                  : nullptr;
-        __nv_bfloat16 dig[7][8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int k = ch * 8 + q;
-            long long X = 0;
-            if (mxb && k < ks.kvalid) {
-                const long long v = x[int64_t(k) * ks.sk];
-                const int ex = int((v >> 52) & 0x7ff);
-                if (ex) {
-                    const long long m = (v & 0xfffffffffffffLL) | (1LL << 52);
-                    const int sh = base_sh - ex;
-                    long long a = 0;
-                    if (sh <= 0) a = m << (-sh);
-                    else if (sh < 63) a = (m + (1LL << (sh - 1))) >> sh;
-                    X = v < 0 ? -a : a;
-                }
-            }
-            // compile-time slice indices keep dig[][] in registers
-#pragma unroll
-            for (int i = 6; i >= 1; --i) {
-                if (i >= slices) continue;
-                int d = int(X & 255);
-                if (d > 128) d -= 256;
-                X = (X - d) >> 8;
-                dig[i][q] = __float2bfloat16_rn(ldexpf(float(d), -8 * i));
-            }
-            dig[0][q] = __float2bfloat16_rn(float(X));
-        }
-        uint8_t* tile0 = out + jb.out_off + int64_t(t) * slices * tile_bytes;
-        const int off = (r >> 3) * 1024 + (r & 7) * 128 + ((ch ^ (r & 7)) << 4);
-#pragma unroll
-        for (int i = 0; i < 7; ++i) {
-            if (i >= slices) continue;
-            uint4 v;
-            __builtin_memcpy(&v, dig[i], 16);
-            *reinterpret_cast<uint4*>(tile0 + int64_t(i) * tile_bytes + off) = v;
-        }
+        long long v[8];
+        pack_load(v, ks, b, jb.row0 + r, live, ch);
+        pack_digits(v, mxb, r, ch, out + jb.out_off + int64_t(t) * slices * tile_bytes, tile_bytes,
+                    slices);
     }
 }
 
@@ -390,7 +387,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
                   const SplitTask* __restrict__ tasks, const uint8_t* __restrict__ apack,
                   const uint8_t* __restrict__ bpack, const int* __restrict__ ea,
-                  const int* __restrict__ eb, Bases b, int slices, int* __restrict__ err) {
+                  const int* __restrict__ eb, const __grid_constant__ Bases b, int slices,
+                  int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // 1024-byte aligned stage ring (the swizzle atom needs it)
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -398,6 +396,9 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
     SplitShared* sh = reinterpret_cast<SplitShared*>(ring + NST * STAGE);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int* serr = &sh->err;
+    // the first item, on its way during the set-up
+    const SplitItem item0 = items[blockIdx.x];
+    const SplitTask task0 = tasks[item0.task];
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < NST; ++i) {
@@ -431,8 +432,12 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
             const bool withhold = blockIdx.x == 0 && atomicCAS(err + 1, 1, 0) == 1;
             uint32_t g = 0;  // global stage counter
             for (int it = blockIdx.x; it < nitems && !*serr; it += gridDim.x) {
-                const SplitItem item = items[it];
-                const SplitTask tk = tasks[item.task];
+                const SplitItem item = it == int(blockIdx.x) ? item0 : items[it];
+                const SplitTask tk = it == int(blockIdx.x) ? task0 : tasks[item.task];
+                // the 8-row atoms that hold rows of the block (the rest of the stage keeps
+                // what was there: it only reaches outputs that are not stored)
+                const uint32_t abytes = uint32_t(min(BM, tk.m - item.mt * BM) + 7) / 8 * 1024;
+                const uint32_t bbytes = uint32_t(min(BN, tk.n - item.nt * BN) + 7) / 8 * 1024;
                 for (int kt = 0; kt < tk.nkt && !*serr; ++kt)
                     for (int t = 0; t < slices; ++t, ++g) {
                         const int st = g % NST;
@@ -440,13 +445,13 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
                         if (!mbar_wait(&sh->empty[st], ph ^ 1, err, serr)) break;
                         if (withhold && g == 0) continue;
                         uint8_t* dst = ring + st * STAGE;
-                        mbar_expect_tx(&sh->full[st], STAGE);
+                        mbar_expect_tx(&sh->full[st], abytes + bbytes);
                         const int64_t ao = tk.a_off + (int64_t(item.mt) * tk.nkt + kt) * slices * A_TILE +
                                            int64_t(t) * A_TILE;
                         const int64_t bo = tk.b_off + (int64_t(item.nt) * tk.nkt + kt) * slices * B_TILE +
                                            int64_t(t) * B_TILE;
-                        bulk_g2s(dst, apack + ao, A_TILE, &sh->full[st]);
-                        bulk_g2s(dst + A_TILE, bpack + bo, B_TILE, &sh->full[st]);
+                        bulk_g2s(dst, apack + ao, abytes, &sh->full[st]);
+                        bulk_g2s(dst + A_TILE, bpack + bo, bbytes, &sh->full[st]);
                     }
             }
             // before the CTA may exit, every copy this thread issued must have landed (in the
@@ -457,21 +462,24 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
-            const uint32_t idesc = idesc_bf16(BM, BN);
             uint32_t g = 0;       // stage counter (matches the producer)
             uint32_t chunk = 0;   // accumulation chunk counter (TMEM double buffer)
             for (int it = blockIdx.x; it < nitems && !*serr; it += gridDim.x) {
-                const SplitItem item = items[it];
-                const SplitTask tk = tasks[item.task];
+                const SplitItem item = it == int(blockIdx.x) ? item0 : items[it];
+                const SplitTask tk = it == int(blockIdx.x) ? task0 : tasks[item.task];
+                // N covers the block's columns (a multiple of 16)
+                const uint32_t idesc = idesc_bf16(BM, (min(BN, tk.n - item.nt * BN) + 15) / 16 * 16);
                 for (int k0 = 0; k0 < tk.nkt && !*serr; k0 += KC, ++chunk) {
                     const int buf = chunk & 1;
                     if (!mbar_wait(&sh->tempty[buf], ((chunk >> 1) & 1) ^ 1, err, serr)) break;
                     asm volatile("tcgen05.fence::after_thread_sync;");
-                    bool first[NACC] = {true, true, true, true};
+                    uint32_t started = 0;  // accumulators written in this chunk
                     const int k1 = min(k0 + KC, tk.nkt);
                     bool ok = true;
                     for (int kt = k0; kt < k1 && ok; ++kt) {
                         const uint32_t g0 = g;
+                        // 16-deep steps with valid k (the others would add zeros)
+                        const int nkk = split_ksteps(tk.kmask, kt);
                         for (int t = 0; t < slices; ++t) {
                             const uint32_t gg = g0 + t;
                             if (!mbar_wait(&sh->full[gg % NST], (gg / NST) & 1, err, serr)) {
@@ -491,11 +499,10 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
                                     const uint32_t sa = smem_u32(ring + ((g0 + ii) % NST) * STAGE);
                                     const uint32_t sb = smem_u32(ring + ((g0 + j) % NST) * STAGE + A_TILE);
                                     const uint32_t td = tmem + uint32_t(buf * NACC * BN + lvl * BN);
-#pragma unroll
-                                    for (int kk = 0; kk < BKT / 16; ++kk) {
+                                    for (int kk = 0; kk < nkk; ++kk) {
                                         mma_bf16(td, sdesc(sa + kk * 32), sdesc(sb + kk * 32), idesc,
-                                                 first[lvl] ? 0u : 1u);
-                                        first[lvl] = false;
+                                                 (started >> lvl) & 1);
+                                        started |= 1u << lvl;
                                     }
                                 }
                             }
@@ -516,14 +523,23 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
         }
     } else {
         // ---------------- epilogue (warps 2..9) ----------------
+        // Two warps per lane quadrant, which take the 16-column groups in turn, so that both
+        // have work on narrow blocks.  c = 0..31 of a warp: group c / 16, column c % 16.
         constexpr int HC = BN / 2;       // columns per epilogue warp
         const int q = warp & 3;          // TMEM lane quadrant of this warp
-        const int h = (warp - 2) >> 2;   // column half
+        const int h = (warp - 2) >> 2;   // first column group
         const int row = q * 32 + lane;   // row of the output tile
         uint32_t chunk = 0;
         for (int it = blockIdx.x; it < nitems && !*serr; it += gridDim.x) {
-            const SplitItem item = items[it];
-            const SplitTask tk = tasks[item.task];
+            const SplitItem item = it == int(blockIdx.x) ? item0 : items[it];
+            const SplitTask tk = it == int(blockIdx.x) ? task0 : tasks[item.task];
+            // the block's columns in this tile (none for a quadrant beyond its rows)
+            const int ncol = q * 32 < tk.m - item.mt * BM ? min(BN, tk.n - item.nt * BN) : 0;
+            const int gr = item.mt * BM + row;
+            const int er = gr < tk.m ? ea[tk.ea_off + gr] : 0;
+            const int ec = lane + 16 * h + 16 * (lane >> 4) < ncol
+                               ? eb[tk.eb_off + item.nt * BN + lane + 16 * h + 16 * (lane >> 4)]
+                               : 0;  // exponent of column c = lane
             float hi[HC], lo[HC];
 #pragma unroll
             for (int c = 0; c < HC; ++c) { hi[c] = 0.f; lo[c] = 0.f; }
@@ -532,36 +548,35 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
                 const int buf = chunk & 1;
                 if (!mbar_wait(&sh->tfull[buf], (chunk >> 1) & 1, err, serr)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;");
-                const uint32_t tbase = tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * NACC * BN + h * HC);
+                const uint32_t tbase = tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * NACC * BN + h * 16);
 #pragma unroll
-                for (int c0 = 0; c0 < HC; c0 += 16) {
+                for (int g = 0; g < 2; ++g) {
+                    if (16 * h + 32 * g >= ncol) continue;
+                    float v[NACC][16];
 #pragma unroll
-                    for (int l = 0; l < NACC; ++l) {
-                        float v[16];
-                        tmem_ld16(tbase + l * BN + c0, v);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    for (int l = 0; l < NACC; ++l) tmem_ld16(tbase + l * BN + 32 * g, v[l]);
+                    tmem_wait(v);
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) df_add(hi[c0 + c], lo[c0 + c], v[c]);
-                    }
+                    for (int l = 0; l < NACC; ++l)
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) df_add(hi[16 * g + c], lo[16 * g + c], v[l][c]);
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sh->tempty[buf]);
             }
             if (!ok) break;
-            const int gr = item.mt * BM + row;
-            if (gr < tk.m) {
-                const int er = ea[tk.ea_off + gr];
-                double* C = b.p[tk.cbuf] + tk.coff;
+            if (ncol == 0) continue;
+            double* C = b.p[tk.cbuf] + tk.coff + gr + int64_t(item.nt * BN) * tk.ldc;
 #pragma unroll
-                for (int c = 0; c < HC; ++c) {
-                    const int gc = item.nt * BN + h * HC + c;
-                    if (gc < tk.n) {
-                        const int ec = eb[tk.eb_off + gc];
-                        const double v = (double(hi[c]) + double(lo[c])) * pow2(er + ec - 16);
-                        double* c = C + gr + int64_t(gc) * tk.ldc;
-                        *c = tk.accum ? *c + v : v;
-                    }
+            for (int c = 0; c < HC; ++c) {
+                const int tc = c % 16 + 16 * h + 32 * (c / 16);
+                if (tc >= ncol) continue;
+                const int e = er + __shfl_sync(0xffffffffu, ec, c) - 16;
+                const double v = scale2(widen(hi[c]) + widen(lo[c]), e);
+                if (gr < tk.m) {
+                    double* out = C + int64_t(tc) * tk.ldc;
+                    *out = tk.accum ? *out + v : v;
                 }
             }
         }
@@ -598,7 +613,7 @@ void launch_split_pack(const PackJob* jobs, int njobs, const KTileSrc* ksrc, con
     }
     const dim3 g(njobs, (max_nkt + KPER - 1) / KPER);
     TN_CUDA(cudaMemsetAsync(gmax, 0, size_t(nrows) * sizeof(unsigned long long), s));
-    split_rowmax_kernel<<<g, PACK_THREADS, 0, s>>>(jobs, ksrc, b, gmax, tile_rows, KPER);
+    split_rowmax_kernel<<<g, PACK_THREADS, 0, s>>>(jobs, ksrc, b, gmax, KPER);
     TN_CUDA(cudaGetLastError());
     split_pack_part_kernel<<<g, PACK_THREADS, 0, s>>>(jobs, ksrc, b, out, expo, gmax, slices,
                                                       tile_rows, KPER);

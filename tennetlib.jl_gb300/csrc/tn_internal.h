@@ -206,7 +206,13 @@ struct PackJob {         // one row tile of one task's operand
 struct SplitTask {
     int64_t coff, a_off, b_off;
     int32_t cbuf, m, n, ldc, nkt, ea_off, eb_off, accum;
+    uint64_t kmask;  // two bits per k tile: 16-deep MMA steps with valid k, less one
 };
+// k tiles that kmask covers; later ones are packed and multiplied whole
+constexpr int SPLIT_KMASK = 32;
+constexpr int split_ksteps(uint64_t kmask, int kt) {
+    return kt < SPLIT_KMASK ? int((kmask >> (2 * kt)) & 3) + 1 : 4;
+}
 struct SplitItem {
     int32_t task, mt, nt, pad;
 };
