@@ -315,7 +315,9 @@ gs_pass_kernel(const __grid_constant__ VecPtrs V, int kk, double* __restrict__ w
         double sum = 0.0;
         for (int bb = lane; bb < (int)gridDim.x; bb += 32)
             sum += reinterpret_cast<volatile double*>(part)[int64_t(j) * gridDim.x + bb];
-        sum = warp_sum(sum);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)  // the butterfly's steps that add no zeros
+            if (o < (int)gridDim.x) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (lane == 0) {
             out[j] = sum;
             if (post.values) post.values[GS_NORM + j] = sum;
@@ -335,109 +337,128 @@ gs_pass_kernel(const __grid_constant__ VecPtrs V, int kk, double* __restrict__ w
 
 // The whole double Gram-Schmidt step of a short residual in one launch:
 //   h1 = V^T w, w -= V h1, h2 = V^T w, w -= V h2, |w|^2, next = w / |w|
-// A cluster of CL CTAs keeps w in registers, each thread one element of up to GS2_PARTS parts of
-// 256 elements; the parts' sums meet through distributed shared memory.  The sums are formed
-// in gs_pass_kernel's order (element, warp, the part's eight warps, parts by lane), so the
-// results are the same bits as its three passes.
+// A cluster of CL CTAs keeps w and the basis in registers, each thread one element of up to
+// gs2_parts(C) parts of 256 elements; the parts' sums meet through distributed shared memory.  A
+// ninth warp posts the results to the host while the others form the next vector.  The sums are
+// formed in gs_pass_kernel's order (element, warp, the part's eight warps, parts by lane; adds
+// of zeros left out), so the results are the same bits as its three passes.
+// Bound by chains of FP64 operations (65 clocks each, the reciprocal root 2000) and the barriers.
 // Three passes and the scaling of the next vector were four launches and at least 34 us for any
-// n; this is one (12-site DMRG run 71 -> 47 ms, 64-site run in split precision 565 -> 440 ms,
-// both with the results posted to the host).  Every CTA sums all parts by itself and FP64 adds
-// are slow, so it is for short vectors (gs2_cluster): from P (2 K + 4) = 256 on (P parts, K
-// vectors) the passes, which spread the parts over all SMs, are as fast.
-constexpr int GS2_PARTS = 4;
+// n; this is one of 9 (n = 250, K = 1) to 25 us (n = 8000, K = 4; 12-site DMRG run 71 -> 47 ms, 64-site run in split precision
+// 565 -> 440 ms, both with the results posted to the host).  Vectors too long for it (gs2_cluster)
+// take the passes, which spread the parts over all SMs.
+constexpr int GS2_THREADS = BLAS_THREADS + 32;
+constexpr int gs2_parts(int C) { return C <= 4 ? 4 : C == 8 ? 3 : C == 16 ? 2 : 1; }
 template <int C>
-__global__ void __launch_bounds__(BLAS_THREADS, 1)
+__global__ void __launch_bounds__(GS2_THREADS, 1)
 gs2_kernel(const __grid_constant__ VecPtrs V, int kk, double* __restrict__ w,
            double* __restrict__ next, int n, double* __restrict__ out, HostPost post) {
     namespace cg = cooperative_groups;
+    constexpr int PARTS = gs2_parts(C), WARPS = BLAS_THREADS / 32;
     cg::cluster_group cl = cg::this_cluster();
-    __shared__ double red[BLAS_THREADS / 32][C];
-    __shared__ double sums[3][GS2_PARTS][C];  // this CTA's parts, one array per phase
-    __shared__ double hs[C];
+    __shared__ double red[WARPS][C];
+    __shared__ double sums[3][PARTS][C];  // this CTA's parts, one array per phase
+    __shared__ double hs[3][C];           // h1, h2, |w|^2
     const int CL = int(cl.num_blocks()), rank = int(cl.block_rank());
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int P = (n + BLAS_THREADS - 1) / BLAS_THREADS;  // part p: CTA p % CL, slot p / CL
-    double x[GS2_PARTS];
+    double x[PARTS], v[PARTS][C];
 #pragma unroll
-    for (int s = 0; s < GS2_PARTS; ++s) {
+    for (int s = 0; s < PARTS; ++s) {
         const int i = (s * CL + rank) * BLAS_THREADS + int(threadIdx.x);
-        x[s] = i < n ? w[i] : 0.0;
+        const bool in = wid < WARPS && i < n;
+        x[s] = in ? w[i] : 0.0;
+#pragma unroll
+        for (int k = 0; k < C; ++k) v[s][k] = in && k < kk ? V.p[k][i] : 0.0;
     }
-    // sums over the parts of phase f for every result, into hs (all CTAs alike)
-    auto finish = [&](int f, int nres) {
-        cl.sync();
-        for (int j = wid; j < nres; j += BLAS_THREADS / 32) {
-            double s = 0.0;
-            if (lane < P) s = cl.map_shared_rank(&sums[f][lane / CL][j], lane % CL)[0];
-            s = warp_sum(s);
-            if (lane == 0) hs[j] = s;
-        }
-        __syncthreads();
-    };
-    auto part_sum = [&](int f, int s, double v, int nres, bool owner, int idx) {
-        if (owner) red[wid][idx] = v;
+    // sum of the part's warps for every result (a barrier before and after)
+    auto part_sum = [&](int f, int s, double r, int nres, bool owner, int idx) {
+        if (wid < WARPS && owner) red[wid][idx] = r;
         __syncthreads();
         if (threadIdx.x < nres) {
-            double sum = 0.0;
+            const int live = (n - (s * CL + rank) * BLAS_THREADS + 31) / 32;  // warps with elements
+            double sum = red[0][threadIdx.x];
 #pragma unroll
-            for (int j = 0; j < BLAS_THREADS / 32; ++j) sum += red[j][threadIdx.x];
+            for (int j = 1; j < WARPS; ++j)
+                if (j < live) sum += red[j][threadIdx.x];
             sums[f][s][threadIdx.x] = sum;
         }
         __syncthreads();
     };
-#pragma unroll 1
+    // sums over the parts of phase f for every result, into hs[f] (all CTAs alike)
+    auto finish = [&](int f, int nres) {
+        if (P == 1) {
+            if (threadIdx.x < nres) hs[f][threadIdx.x] = sums[f][0][threadIdx.x];
+            __syncthreads();
+            return;
+        }
+        cl.sync();
+        if (wid < WARPS)
+            for (int j = wid; j < nres; j += WARPS) {
+                double s = 0.0;
+                if (lane < P) s = cl.map_shared_rank(&sums[f][lane / CL][j], lane % CL)[0];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)  // the butterfly's steps that add no zeros
+                    if (o < P) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) hs[f][j] = s;
+            }
+        __syncthreads();
+    };
+#pragma unroll
     for (int f = 0; f < 2; ++f) {
 #pragma unroll
-        for (int s = 0; s < GS2_PARTS; ++s) {
-            if (s * CL + rank >= P) break;
-            const int i = (s * CL + rank) * BLAS_THREADS + int(threadIdx.x);
+        for (int s = 0; s < PARTS; ++s) {
+            if (s * CL + rank >= P) continue;
             double acc[C];
 #pragma unroll
-            for (int k = 0; k < C; ++k) acc[k] = (k < kk && i < n) ? fma(V.p[k][i], x[s], 0.0) : 0.0;
-            const double v = warp_sum_multi<C>(acc, lane);
-            part_sum(f, s, v, kk, warp_sum_owner<C>(lane), warp_sum_index<C>(lane));
+            for (int k = 0; k < C; ++k) acc[k] = k < kk ? v[s][k] * x[s] : 0.0;
+            const double r = warp_sum_multi<C>(acc, lane);
+            part_sum(f, s, r, kk, warp_sum_owner<C>(lane), warp_sum_index<C>(lane));
         }
         finish(f, kk);
-        if (rank == 0 && threadIdx.x < kk) {
-            const double h = hs[threadIdx.x];
-            out[f * GS_H2 + threadIdx.x] = h;
-            post.values[f * GS_H2 + threadIdx.x] = h;
-        }
 #pragma unroll
-        for (int s = 0; s < GS2_PARTS; ++s) {
-            const int i = (s * CL + rank) * BLAS_THREADS + int(threadIdx.x);
-            if (i < n)
-                for (int k = 0; k < kk; ++k) x[s] = fma(-hs[k], V.p[k][i], x[s]);
+        for (int s = 0; s < PARTS; ++s) {
+            if (s * CL + rank >= P) continue;
+#pragma unroll
+            for (int k = 0; k < C; ++k)
+                if (k < kk) x[s] = fma(-hs[f][k], v[s][k], x[s]);
         }
-        __syncthreads();  // hs is read until here
     }
 #pragma unroll
-    for (int s = 0; s < GS2_PARTS; ++s) {
-        if (s * CL + rank >= P) break;
-        const double v = warp_sum(fma(x[s], x[s], 0.0));
-        part_sum(2, s, v, 1, lane == 0, 0);
+    for (int s = 0; s < PARTS; ++s) {
+        if (s * CL + rank >= P) continue;
+        part_sum(2, s, warp_sum(x[s] * x[s]), 1, lane == 0, 0);
     }
     finish(2, 1);
-    const double nrm = hs[0];
-    const double scale = 1.0 / sqrt(nrm);
+    if (wid < WARPS) {
+        const double scale = next ? 1.0 / sqrt(hs[2][0]) : 0.0;
 #pragma unroll
-    for (int s = 0; s < GS2_PARTS; ++s) {
-        const int i = (s * CL + rank) * BLAS_THREADS + int(threadIdx.x);
-        if (i < n) {
-            w[i] = x[s];
-            if (next) next[i] = x[s] * scale;
+        for (int s = 0; s < PARTS; ++s) {
+            const int i = (s * CL + rank) * BLAS_THREADS + int(threadIdx.x);
+            if (s * CL + rank < P && i < n) {
+                w[i] = x[s];
+                if (next) next[i] = x[s] * scale;
+            }
         }
-    }
-    if (rank == 0) {
-        if (threadIdx.x == 0) {
-            out[GS_NORM] = nrm;
-            post.values[GS_NORM] = nrm;
+        if (rank == 0 && threadIdx.x < kk) {
+            out[threadIdx.x] = hs[0][threadIdx.x];
+            out[GS_H2 + threadIdx.x] = hs[1][threadIdx.x];
+            if (threadIdx.x == 0) out[GS_NORM] = hs[2][0];
+        }
+    } else if (rank == 0) {
+        if (lane < kk) {
+            post.values[lane] = hs[0][lane];
+            post.values[GS_H2 + lane] = hs[1][lane];
+        }
+        if (lane == 0) {
+            post.values[GS_NORM] = hs[2][0];
             if (post.start) post.values[GS_START] = *post.start;
         }
-        __syncthreads();
-        host_post(post);
+        __syncwarp();
+        __threadfence_system();
+        if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(post.flag) = post.seq;
     }
-    cl.sync();  // the other CTAs read this one's sums until here
+    if (P > 1) cl.sync();  // the other CTAs read this one's sums until here
 }
 
 __global__ void __launch_bounds__(BLAS_THREADS)
@@ -536,10 +557,15 @@ void launch_gs_pass(const double* const* V, int K, double* w, const double* hin,
     count_krylov_bytes(int64_t(1 + ((hin || !norm) ? K : 0) + (hin ? 1 : 0)) * n * 8);
 }
 
-// CTAs of gs2_kernel's cluster for n elements and K vectors, 0: too long for it
+// CTAs of gs2_kernel's cluster for n elements and K vectors, 0: too long for it.  A CTA's parts
+// come one after the other, so the line is where they take as long as the passes (back-to-back
+// launches): K = 4: 24.6 against 25.6 us at four parts per CTA (n = 8000) and 33 against 27 at
+// six; K = 8: 21.5 against 27.7 at two and 33 against 29 at four; K = 16: 29 against 34 at two
+// and 49 against 35 at four; K = 24: 27 against 43 at one and 45 against 45 at two.
 static int gs2_cluster(int64_t n, int K) {
     const int64_t P = (n + BLAS_THREADS - 1) / BLAS_THREADS;
-    if (P < 1 || P > 8 * GS2_PARTS || P * (2 * K + 4) > 256) return 0;
+    const int parts = gs2_parts(K <= 4 ? 4 : K <= 8 ? 8 : K <= 16 ? 16 : 32);
+    if (P < 1 || P > 8 * parts) return 0;
     int c = 1;
     while (c < 8 && c < P) c *= 2;
     return c;
@@ -557,7 +583,7 @@ void launch_gs2(const double* const* V, int K, double* w, double* next, int64_t 
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(c));
-    cfg.blockDim = dim3(BLAS_THREADS);
+    cfg.blockDim = dim3(GS2_THREADS);
     cfg.stream = s;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
