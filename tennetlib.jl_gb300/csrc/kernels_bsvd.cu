@@ -10,7 +10,9 @@
 //    memory (double-float), the trailing matrix is updated by grouped GEMMs with the compact
 //    WY form Q_p = I - V T V^T (Schreiber & Van Loan 1989);
 //  * one-sided Jacobi on R^T (Drmac & Veselic 2008: the triangular factor makes the cyclic
-//    method converge in a few sweeps) by rounds of column-block pairs: in every round each CTA
+//    method converge in a few sweeps) by rounds of column-block pairs (the FP32 presolve on the
+//    pairs' Gram matrices, bj32_kernel; the double-float polish and longer columns column by
+//    column, bj_kernel): in every round each CTA
 //    of a matrix's group takes one pair of 16-column blocks (8 in double-float), stages the
 //    columns of X and V in shared memory and rotates every column pair across the two blocks;
 //    the pairs of one round are disjoint (round-robin tournament over the blocks), and the
@@ -748,6 +750,279 @@ bj_kernel(const BjDesc* __restrict__ descs, int nd, float tol, int max_sweeps, i
     if (lc == 0 && threadIdx.x == 0 && d.sweeps) *d.sweeps = sweep;
 }
 
+// ------------------------------------------------------------------------------------
+// FP32 presolve by block pairs
+//
+// Same rounds of block pairs and the same rotations as bj_kernel, but a task of 16 + 16 columns
+// forms its 32 x 32 Gram matrix once, runs the rotations of its 16 rounds of disjoint pairs on
+// that matrix (two-sided, in shared memory) while collecting their product W, and then applies W
+// to the columns of X and V as one 32 x 32 product per row.  bj_kernel read and wrote every
+// staged column in every one of the 16 sub-rounds, behind block-wide reductions: 85000 clocks per
+// task whatever the length, 16 x (reduction + angle + barriers) of it latency.  Here a sub-round
+// is 2 x 2 blocks of a small matrix and one barrier.  The first round of a sweep runs all 31 rounds
+// of the 32 columns instead, which covers the pairs inside the blocks.  The Gram matrix is good to
+// ~1e-6 of the columns' norms, the rotation threshold is 2e-5; what it misses the next sweep sees.
+// Columns of the pair are staged with a stride of an odd number of float4, and a Gram tile
+// takes columns 8 apart, so that a quarter-warp's 16-byte reads hit different banks.
+// Measured, with the CTAs shared out by time (bsvd.cpp): the presolve of a chi = 2048 bond (seven
+// blocks up to 1077 x 994) 29 -> 14 ms, a task of n = 991 85000 -> 55000 clocks (Gram 11000, rounds
+// 13000, products 25000, staging 10000).
+// ------------------------------------------------------------------------------------
+constexpr int PB = 16, PC = 2 * PB;            // columns of a block, of a pair
+constexpr int BJ32_MAXN = 1280;                // longest columns (shared memory)
+constexpr int GRAM_TILES = 36, GRAM_GROUPS = BT / GRAM_TILES;  // 4 x 4 tiles (upper), row groups
+__host__ __device__ constexpr int bj32_ld(int n) { return 4 * (((n + 3) / 4) | 1); }
+constexpr size_t bj32_smem(int n) {
+    return size_t(PC) * bj32_ld(n) * 4 + size_t(GRAM_GROUPS) * GRAM_TILES * 16 * 4;
+}
+
+// rotation of a pair with squared norms a, b and inner product g (identity below the threshold)
+struct Turn {
+    float c, s, t;
+    bool on;
+};
+// Approximate roots and quotients (about 2^-22): an angle only has to shrink the pair's cosine,
+// which the next sweep measures again, and c and s belong to one t, so W is orthogonal to FP32
+// rounding.
+__device__ __forceinline__ Turn bj32_turn(float a, float b, float g, float tol) {
+    Turn r{1.f, 0.f, 0.f, false};
+    // columns below 1e-36 (2e-18 of the largest value) are left alone, as in bj_kernel
+    if (!(a > 1e-36f && b > 1e-36f)) return r;
+    const float ra = rsqrtf(a), rb = rsqrtf(b), cosine = g * ra * rb;
+    if (!(fabsf(cosine) > tol)) return r;
+    // tan = h / (d + sign(d) sqrt(d^2 + h^2)) with d = b - a and h = 2 g, both over sqrt(a b)
+    // (d stays below 1e19, h within [2 tol, 2]: no overflow of the squares)
+    const float d = (b - a) * ra * rb, h = 2.f * cosine;
+    const float w = fmaf(d, d, h * h);
+    const float t = __fdividef(h, d + copysignf(w * rsqrtf(w), d));
+    const float c = rsqrtf(fmaf(t, t, 1.f));
+    return Turn{c, c * t, t, true};
+}
+
+__global__ void __launch_bounds__(BT, 1)
+bj32_kernel(const BjDesc* __restrict__ descs, int nd, float tol, int max_sweeps,
+            int* __restrict__ err) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ float G[2][PC][PC + 1];
+    __shared__ __align__(16) float Wm[PC][PC + 4];
+    __shared__ float4 turns[PB];  // c, s and the columns of a round's pairs
+    __shared__ int goff[PC];      // offsets of the pair's columns, -1: none
+    __shared__ int s_rot, s_task, s_fail;
+    int di = 0;
+    while (di < nd && !(int(blockIdx.x) >= descs[di].cta0 &&
+                        int(blockIdx.x) < descs[di].cta0 + descs[di].ncta))
+        ++di;
+    if (di >= nd) return;
+    const BjDesc d = descs[di];
+    const int lc = int(blockIdx.x) - d.cta0, n = d.n, ld = bj32_ld(n), nq = (n + 3) / 4;
+    float* Xs = reinterpret_cast<float*>(smem);
+    float* red = Xs + PC * ld;
+    float* X = static_cast<float*>(d.X);
+    float* V = static_cast<float*>(d.V);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        s_rot = 0;
+        // test hook (tn_ctx_inject_wait_timeout, code 2), as in bj_kernel
+        s_fail = (di == 0 && lc == 0 && atomicCAS(err + 1, 2, 0) == 2) ? 1 : 0;
+    }
+    __syncthreads();
+    if (s_fail) return;
+    int ti = 0, tj = tid % GRAM_TILES;  // this thread's Gram tile, ti <= tj
+    while (tj >= 8 - ti) {
+        tj -= 8 - ti;
+        ++ti;
+    }
+    tj += ti;
+    const int group = tid / GRAM_TILES;
+
+    // the pair's columns of X or V: two columns per warp, sixteen loads in flight
+    auto stage = [&](const float* src) {
+        const int o0 = goff[warp], o1 = goff[warp + BT / 32];
+        float* x0 = Xs + warp * ld;
+        float* x1 = x0 + BT / 32 * ld;
+        for (int i0 = lane; i0 < 4 * nq; i0 += 256) {
+            float a[8], b[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int i = i0 + 32 * u;
+                a[u] = o0 >= 0 && i < n ? __ldcg(src + o0 + i) : 0.f;
+                b[u] = o1 >= 0 && i < n ? __ldcg(src + o1 + i) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int i = i0 + 32 * u;
+                if (i < 4 * nq) {
+                    x0[i] = a[u];
+                    x1[i] = b[u];
+                }
+            }
+        }
+    };
+    // dst <- staged columns times W: 8 rows (32 apart) x 8 columns per thread, so that a value read
+    // from shared memory is used eight times: an LDS.128 takes four clocks of the SM even when
+    // all lanes read the same 16 bytes (one row per thread with W by broadcasts took 70000 clocks)
+    auto apply = [&](float* dst) {
+        const int c0 = (warp & 3) * 8;
+        for (int r0 = (warp >> 2) * 256 + lane; r0 - lane < n; r0 += 1024) {
+            float acc[8][8] = {};
+#pragma unroll 2
+            for (int k = 0; k < PC; ++k) {
+                const float* xk = Xs + k * ld;
+                float x[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) x[r] = r0 + 32 * r < n ? xk[r0 + 32 * r] : 0.f;
+                const float4 w0 = *reinterpret_cast<const float4*>(&Wm[k][c0]);
+                const float4 w1 = *reinterpret_cast<const float4*>(&Wm[k][c0 + 4]);
+                const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(x[r], w[c], acc[r][c]);
+            }
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const int o = goff[c0 + c];
+                if (o < 0) continue;
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                    if (r0 + 32 * r < n) dst[o + r0 + 32 * r] = acc[r][c];
+            }
+        }
+    };
+
+    auto task = [&](int I, int J, bool full) {
+        if (tid < PC) {
+            const int g = (tid < PB ? I : J) * PB + tid % PB;
+            goff[tid] = (tid < PB || J < d.nb) && g < n ? g * n : -1;
+        }
+        if (tid == 0) s_task = 0;
+        __syncthreads();
+        stage(X);
+        for (int e = tid; e < PC * PC; e += BT) Wm[e / PC][e % PC] = e / PC == e % PC ? 1.f : 0.f;
+        __syncthreads();
+        // Gram matrix: tile (ti, tj) holds columns ti + 8 a and tj + 8 b
+        if (group < GRAM_GROUPS) {
+            float acc[4][4] = {};
+            for (int q = group; q < nq; q += GRAM_GROUPS) {
+                float4 xa[4], xb[4];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    xa[a] = *reinterpret_cast<const float4*>(Xs + (ti + 8 * a) * ld + 4 * q);
+                    xb[a] = *reinterpret_cast<const float4*>(Xs + (tj + 8 * a) * ld + 4 * q);
+                }
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        acc[a][b] = fmaf(xa[a].x, xb[b].x, acc[a][b]);
+                        acc[a][b] = fmaf(xa[a].y, xb[b].y, acc[a][b]);
+                        acc[a][b] = fmaf(xa[a].z, xb[b].z, acc[a][b]);
+                        acc[a][b] = fmaf(xa[a].w, xb[b].w, acc[a][b]);
+                    }
+            }
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+                *reinterpret_cast<float4*>(red + (tid * 4 + a) * 4) =
+                    make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+        }
+        __syncthreads();
+        for (int e = tid; e < GRAM_TILES * 16; e += BT) {
+            int p = 0, q = e / 16;
+            while (q >= 8 - p) {
+                q -= 8 - p;
+                ++p;
+            }
+            q += p;
+            float s = 0.f;
+            for (int g = 0; g < GRAM_GROUPS; ++g) s += red[g * GRAM_TILES * 16 + e];
+            const int ca = p + 8 * (e % 16 / 4), cb = q + 8 * (e % 4);
+            G[0][ca][cb] = s;
+            G[0][cb][ca] = s;
+        }
+        __syncthreads();
+        // rounds of 16 disjoint pairs on the Gram matrix: one warp forms the angles (formed by
+        // every warp, they took 1200 clocks a round), then 2 x 2 blocks of two pairs and columns
+        // of W
+        int cur = 0;
+        const int rounds = full ? PC - 1 : PB;
+        for (int k = 0; k < rounds; ++k, cur ^= 1) {
+            const float(&g)[PC][PC + 1] = G[cur];
+            float(&o)[PC][PC + 1] = G[cur ^ 1];
+            if (tid < PB) {
+                int i = tid, j = PB + (tid + k) % PB;
+                if (full) {
+                    const int x = rr_player(PC, k, tid), y = rr_player(PC, k, PC - 1 - tid);
+                    i = min(x, y);
+                    j = max(x, y);
+                }
+                const float a = g[i][i], b = g[j][j], x = g[i][j];
+                const Turn T = bj32_turn(a, b, x, tol);
+                turns[tid] = make_float4(T.c, T.s, __int_as_float(i), __int_as_float(j));
+                o[i][i] = a - T.t * x;
+                o[j][j] = b + T.t * x;
+                o[i][j] = o[j][i] = T.on ? 0.f : x;
+                if (T.on) s_task = 1;
+            }
+            __syncthreads();
+            const float4 A = turns[(tid / PB) % PB];  // rows of the block, or the columns of W
+            const int ia = __float_as_int(A.z), ja = __float_as_int(A.w);
+            if (tid < PB * PB) {
+                const float4 B = turns[tid % PB];
+                const int ib = __float_as_int(B.z), jb = __float_as_int(B.w);
+                if (tid / PB != tid % PB) {
+                    const float g11 = g[ia][ib], g12 = g[ia][jb], g21 = g[ja][ib], g22 = g[ja][jb];
+                    const float h11 = A.x * g11 - A.y * g21, h12 = A.x * g12 - A.y * g22;
+                    const float h21 = A.y * g11 + A.x * g21, h22 = A.y * g12 + A.x * g22;
+                    o[ia][ib] = B.x * h11 - B.y * h12;
+                    o[ia][jb] = B.y * h11 + B.x * h12;
+                    o[ja][ib] = B.x * h21 - B.y * h22;
+                    o[ja][jb] = B.y * h21 + B.x * h22;
+                }
+            } else {  // W <- W J, two rows
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int row = lane % PB + PB * h;
+                    const float x = Wm[row][ia], y = Wm[row][ja];
+                    Wm[row][ia] = A.x * x - A.y * y;
+                    Wm[row][ja] = A.y * x + A.x * y;
+                }
+            }
+            __syncthreads();
+        }
+        if (!s_task) return;  // uniform: read after the last round's barrier
+        if (tid == 0) s_rot = 1;
+        apply(X);
+        __syncthreads();
+        stage(V);
+        __syncthreads();
+        apply(V);
+        __syncthreads();  // Xs, Wm and goff are read until here
+    };
+
+    const int nbe = d.nb + (d.nb & 1);
+    unsigned nbar = 0;
+    int sweep = 0;
+    for (sweep = 0; sweep < max_sweeps; ++sweep) {
+        if (lc == 0 && tid == 0) d.flags[(sweep + 1) % 3] = 0;
+        for (int r = 0; r < max(nbe - 1, 1); ++r) {
+            for (int t = lc; t < nbe / 2; t += d.ncta) {
+                const int p = rr_player(nbe, r, t), q = rr_player(nbe, r, nbe - 1 - t);
+                const int I = min(p, q), J = max(p, q);
+                if (J >= d.nb && r > 0) continue;  // alone: its own pairs in the first round only
+                task(I, J, r == 0);
+                __syncthreads();
+                if (tid == 0 && s_rot) {
+                    atomicOr(&d.flags[sweep % 3], 1);
+                    s_rot = 0;
+                }
+            }
+            if (!group_barrier(d.bar, (++nbar) * unsigned(d.ncta), err, &s_fail)) return;
+        }
+        if (!*reinterpret_cast<volatile int*>(&d.flags[sweep % 3])) break;
+    }
+    if (lc == 0 && tid == 0 && d.sweeps) *d.sweeps = sweep;
+}
+
 // singular values = column norms of Y (double-float), sorted descending with the
 // permutation (PY = P Y and QV = [V; 0] are written by bsvd_outputs_kernel)
 __global__ void __launch_bounds__(BT) bsvd_finish_kernel(const BsvdBlk* __restrict__ descs,
@@ -857,6 +1132,9 @@ int bsvd_panel_width(int mmax) {
 // double-float: B in {16, 8, 4, 2}, the polish with half the FP32 width or more).
 int bsvd_max_n() { return 3568; }
 
+// The FP32 presolve takes bj32_kernel while its staged columns fit shared memory
+static bool use_bj32(int maxn, int precision) { return precision == 0 && maxn <= BJ32_MAXN; }
+
 static int bj_block(int maxn, int precision) {
     const int rm = precision == 0 ? JRegs<float>::RM : JRegs<df2>::RM;
     const int esz = precision == 0 ? 4 : 8;
@@ -903,9 +1181,21 @@ void launch_bsvd_elem(const BsvdBlk* d, int nb, int64_t nnmax, int op, double* a
     count_launch();
 }
 
-int bsvd_jacobi_block(int maxn, int precision) { return bj_block(maxn, precision); }
+int bsvd_jacobi_block(int maxn, int precision) {
+    return use_bj32(maxn, precision) ? PB : bj_block(maxn, precision);
+}
 
 int bsvd_jacobi_capacity(int maxn, int precision) {
+    if (use_bj32(maxn, precision)) {
+        const size_t shm = bj32_smem(maxn);
+        TN_CUDA(cudaFuncSetAttribute(bj32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(shm)));
+        int dev = 0, nsm = 0, per = 0;
+        TN_CUDA(cudaGetDevice(&dev));
+        TN_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        TN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, bj32_kernel, BT, shm));
+        return nsm * per;
+    }
     switch (bsvd_jacobi_block(maxn, precision) + 100 * precision) {
         case 16: return bj_capacity<float, 16>(maxn);
         case 8: return bj_capacity<float, 8>(maxn);
@@ -924,6 +1214,18 @@ void launch_bsvd_jacobi(const BjDesc* d, int nd, int nctas, int maxn, int precis
     TN_REQUIRE(maxn <= bsvd_max_n(), "block SVD: block too large for the Jacobi kernel");
     // rotation threshold above the rounding noise of a double-float dot product
     const float tdf = 3.55e-15f * sqrtf(float(maxn > 1 ? maxn : 1)) * 32.f;
+    if (use_bj32(maxn, precision)) {
+        const size_t shm = bj32_smem(maxn);
+        TN_CUDA(cudaFuncSetAttribute(bj32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(shm)));
+        float tol = 2.0e-5f;
+        int max_sweeps = 30;
+        void* args[] = {(void*)&d, (void*)&nd, (void*)&tol, (void*)&max_sweeps, (void*)&err};
+        TN_CUDA(cudaLaunchCooperativeKernel((const void*)bj32_kernel, dim3(nctas), dim3(BT), args,
+                                            shm, s));
+        count_launch();
+        return;
+    }
     switch (bsvd_jacobi_block(maxn, precision) + 100 * precision) {
         case 16: bj_launch<float, 16>(d, nd, nctas, maxn, 2.0e-5f, 30, 0, err, s); break;
         case 8: bj_launch<float, 8>(d, nd, nctas, maxn, 2.0e-5f, 30, 0, err, s); break;

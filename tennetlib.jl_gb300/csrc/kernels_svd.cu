@@ -1337,6 +1337,8 @@ void launch_svd_extract_complex(const ExtractDesc* d, int nb, const double* QV, 
     count_launch();
 }
 
+bool svd_size_class(int m, int n) { return m <= FAST_M && n <= FAST_N; }
+
 void launch_svd_jacobi(const SvdBlockDesc* d, int nb, int max_n, const double* src, double* X,
                        double* W, double* V, double* P, double* S, int* perm, int* sweeps_out,
                        cudaStream_t s) {

@@ -315,6 +315,8 @@ struct SvdBlockDesc {
     int64_t s_off;     // offset of the singular values (n) and permutation
     int32_t rows, cols, m, n, trans, pad;
 };
+// whether the one-CTA kernel has a size class for an m x n work matrix (m >= n)
+bool svd_size_class(int m, int n);
 void launch_svd_jacobi(const SvdBlockDesc* d, int nb, int max_n, const double* src, double* X,
                        double* W, double* V, double* P, double* S, int* perm, int* sweeps_out,
                        cudaStream_t s);
