@@ -9,6 +9,7 @@
 //  * leg permutation (move one leg of a tensor to the end and back) and small helpers.
 #include <cuda_runtime.h>
 
+#include "reduce.cuh"
 #include "ttn_internal.h"
 
 namespace tn {
@@ -61,10 +62,16 @@ bgs_pass_kernel(const BGsDesc* __restrict__ descs, double sign, int dots, int no
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nres = (dots ? kk : 0) + (norm ? 1 : 0);
+    if (dots) {
+        double t[K];
 #pragma unroll
-    for (int k = 0; k <= K; ++k) {
-        const double v = warp_sum(acc[k]);
-        if (lane == 0) red[wid][k] = v;
+        for (int k = 0; k < K; ++k) t[k] = acc[k];
+        const double v = warp_sum_multi<K>(t, lane);
+        if (warp_sum_owner<K>(lane)) red[wid][warp_sum_index<K>(lane)] = v;
+    }
+    if (norm) {
+        const double v = warp_sum(acc[K]);
+        if (lane == 0) red[wid][K] = v;
     }
     __syncthreads();
     double* part = part_all + int64_t(blockIdx.y) * (BK_MAX + 1) * gridDim.x;
@@ -441,10 +448,19 @@ __device__ __forceinline__ bool inst_barrier(unsigned* bar, unsigned target, int
 // then updates its rows.  Partials and the published row are double-buffered by column parity:
 // a CTA can only reuse a buffer after the next barrier, which every CTA reaches only once it
 // has read the totals of the previous column.
+//
+// Bound by the FP64 pipe and the chain of a column (sums, barrier, totals, root and divisions,
+// update), not by memory.  A warp-wide FP64 operation takes 64 clocks, so a thread works on 8
+// columns of one row (4 column groups x 2 groups of 32 rows per CTA, 64 rows in flight), warp sums
+// are merged (9 adds for 8 columns instead of 40), and the two divisions of the reflector go to
+// two warps.  With one row of 32 columns per thread and plain butterflies (160 adds) a panel of
+// four 4096 x 64 matrices took 658 us, now 315 (four 64-site trees at chi = 64: 751 -> 675 ms a sweep).
+constexpr int HP_COLS = 8, HP_CG = HH_B / HP_COLS, HP_RG = BT / 32 / HP_CG;
+constexpr int HP_ROWS = 32 * HP_RG;  // rows of a CTA in one pass
 __global__ void __launch_bounds__(BT, 2)
 hh_panel_coop_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* err) {
     constexpr int W1 = HH_B + 1;
-    __shared__ double red[BT / 32][W1];
+    __shared__ double red[HP_RG][W1];
     __shared__ double tot[W1];
     __shared__ double wsh[HH_B];
     __shared__ double sc[3];
@@ -469,85 +485,89 @@ hh_panel_coop_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* e
     double* parts = D.part;                          // 2 x G x W1: [sigma^2, s_0, s_1, ...]
     double* pubs = D.part + 2 * int64_t(G) * W1;     // 2 x W1: A[j, j], A[j, j+1], ...
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int cg = wid % HP_CG, rg = wid / HP_CG, c0 = cg * HP_COLS;
     unsigned nb = 0;
     for (int j = p0; j < pe; ++j) {
         const int buf = j & 1;
         double* col = D.A + int64_t(j) * m;
         const int nk = pe - j - 1;
+        const bool mine = c0 < nk;  // this warp's column group has columns
         double ss = 0.0;
-        double acc[HH_B];
+        double acc[HP_COLS];
 #pragma unroll
-        for (int c = 0; c < HH_B; ++c) acc[c] = 0.0;
-        for (int64_t i = (r0 > j + 1 ? r0 : j + 1) + threadIdx.x; i < r1; i += BT) {
-            const double x = col[i];
-            ss = fma(x, x, ss);
-            const double* arow = D.A + i + int64_t(j + 1) * m;
-            // groups of 8 columns past nk are skipped whole
+        for (int c = 0; c < HP_COLS; ++c) acc[c] = 0.0;
+        if (mine || cg == 0)
+            for (int64_t i = r0 + 32 * rg + lane; i < r1; i += HP_ROWS) {
+                if (i <= j) continue;
+                const double x = col[i];
+                if (cg == 0) ss = fma(x, x, ss);
+                const double* arow = D.A + i + int64_t(j + 1 + c0) * m;
 #pragma unroll
-            for (int cg = 0; cg < HH_B; cg += 8) {
-                if (cg >= nk) break;
-#pragma unroll
-                for (int c = cg; c < cg + 8; ++c)
-                    if (c < nk) acc[c] = fma(x, arow[int64_t(c) * m], acc[c]);
+                for (int c = 0; c < HP_COLS; ++c)
+                    if (c0 + c < nk) acc[c] = fma(x, arow[int64_t(c) * m], acc[c]);
             }
+        if (cg == 0) {
+            ss = warp_sum(ss);
+            if (lane == 0) red[rg][0] = ss;
         }
-        ss = warp_sum(ss);
-        if (lane == 0) red[wid][0] = ss;
-#pragma unroll
-        for (int c = 0; c < HH_B; ++c) {
-            if (c >= ((nk + 7) & ~7)) break;
-            const double v = warp_sum(acc[c]);
-            if (lane == 0) red[wid][1 + c] = v;
+        if (mine) {
+            const double v = warp_sum_multi<HP_COLS>(acc, lane);
+            if (warp_sum_owner<HP_COLS>(lane)) red[rg][1 + c0 + warp_sum_index<HP_COLS>(lane)] = v;
         }
         __syncthreads();
         if (threadIdx.x <= nk) {
-            double t = 0.0;
-            for (int w = 0; w < BT / 32; ++w) t += red[w][threadIdx.x];
+            double t = red[0][threadIdx.x];
+#pragma unroll
+            for (int w = 1; w < HP_RG; ++w) t += red[w][threadIdx.x];
             parts[(int64_t(buf) * G + g) * W1 + threadIdx.x] = t;
             if (j >= r0 && j < r1) pubs[buf * W1 + threadIdx.x] = col[j + int64_t(threadIdx.x) * m];
         }
         if (!inst_barrier(D.bar, (++nb) * unsigned(G), err, &s_fail)) return;
         // totals: every CTA sums the G partials in the same fixed order (lane-strided, then a
-        // warp tree), so the reflectors are identical everywhere
+        // warp tree), four results per warp, so the reflectors are identical everywhere
         // (L2 loads: the partials were written by other SMs before the barrier's fences)
         const double* pall = parts + int64_t(buf) * G * W1;
         const double* pub = pubs + buf * W1;
-        for (int c = wid; c <= nk; c += BT / 32) {
-            double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
-            int b = lane;
-            for (; b + 96 < G; b += 128) {
-                t0 += __ldcg(pall + int64_t(b) * W1 + c);
-                t1 += __ldcg(pall + int64_t(b + 32) * W1 + c);
-                t2 += __ldcg(pall + int64_t(b + 64) * W1 + c);
-                t3 += __ldcg(pall + int64_t(b + 96) * W1 + c);
-            }
-            for (; b < G; b += 32) t0 += __ldcg(pall + int64_t(b) * W1 + c);
-            const double t = warp_sum((t0 + t1) + (t2 + t3));
-            if (lane == 0) tot[c] = t;
+        static_assert(4 * (BT / 32) >= HH_B, "a panel column has at most HH_B totals");
+        if (4 * wid <= nk) {
+            double t[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int b = lane; b < G; b += 32)
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (4 * wid + u <= nk) t[u] += __ldcg(pall + int64_t(b) * W1 + 4 * wid + u);
+            const double v = warp_sum_multi<4>(t, lane);
+            if (warp_sum_owner<4>(lane)) tot[4 * wid + warp_sum_index<4>(lane)] = v;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            double tau, scale, beta;
-            make_reflector(__ldcg(pub), tot[0], tau, scale, beta);
-            sc[0] = tau;
-            sc[1] = scale;
-            sc[2] = beta;
+        if (threadIdx.x == 0 || threadIdx.x == 32) {  // two warps, one division each
+            const double alpha = __ldcg(pub), sig = tot[0];
+            const bool zero = sig == 0.0;
+            const double nrm = sqrt(alpha * alpha + sig);
+            const double beta = zero ? alpha : (alpha >= 0.0 ? -nrm : nrm);
+            if (threadIdx.x == 0) {
+                sc[0] = zero ? 0.0 : (beta - alpha) / beta;
+                sc[2] = beta;
+            } else {
+                sc[1] = zero ? 0.0 : 1.0 / (alpha - beta);
+            }
         }
         __syncthreads();
         const double tau = sc[0], scale = sc[1], beta = sc[2];
         if (threadIdx.x < nk) wsh[threadIdx.x] = tau * (__ldcg(pub + 1 + threadIdx.x) + scale * tot[1 + threadIdx.x]);
         __syncthreads();
-        const int64_t i0 = r0 > j ? r0 : j;
-        if (nk > 0) {
-            for (int64_t i = i0 + threadIdx.x; i < r1; i += BT) {
+        if (mine)
+            for (int64_t i = r0 + 32 * rg + lane; i < r1; i += HP_ROWS) {
+                if (i < j) continue;
                 const double v = i == j ? 1.0 : col[i] * scale;
-                for (int c = 0; c < nk; ++c) {
-                    double* a = D.A + i + int64_t(j + 1 + c) * m;
-                    *a = fma(-v, wsh[c], *a);
-                }
+                double* arow = D.A + i + int64_t(j + 1 + c0) * m;
+#pragma unroll
+                for (int c = 0; c < HP_COLS; ++c)
+                    if (c0 + c < nk) arow[int64_t(c) * m] = fma(-v, wsh[c0 + c], arow[int64_t(c) * m]);
             }
-        }
-        for (int64_t i = i0 + threadIdx.x; i < r1; i += BT) col[i] = i == j ? beta : col[i] * scale;
+        __syncthreads();  // every column group has read column j
+        if (cg == 0)
+            for (int64_t i = r0 + 32 * rg + lane; i < r1; i += HP_ROWS)
+                if (i >= j) col[i] = i == j ? beta : col[i] * scale;
         if (g == 0 && threadIdx.x == 0) D.tau[j] = tau;
         __syncthreads();
     }
@@ -801,6 +821,8 @@ void launch_hh_column(const HhDesc* d, int ninst, int64_t mmax, int j, int p0, i
 }
 
 // co-resident CTAs of the cooperative panel kernel on the current device (cached per device)
+int hh_coop_rows() { return HP_ROWS; }
+
 int hh_coop_capacity() {
     constexpr int MAXDEV = 64;
     static int cap[MAXDEV] = {};

@@ -1226,7 +1226,7 @@ void run_qr_move(TtnGroup& G, int v, int u, int maxdim, int mindim = 1, double c
             int used = 0;
             for (auto& h : hh) {
                 h.ncta = std::max(1, int(double(cap - nh0) * double(h.m) / tot));
-                h.ncta = int(std::min<int64_t>(h.ncta, std::max<int64_t>(1, (h.m + 255) / 256)));
+                h.ncta = int(std::min<int64_t>(h.ncta, (h.m + hh_coop_rows() - 1) / hh_coop_rows()));
                 h.cta0 = used;
                 used += h.ncta;
             }

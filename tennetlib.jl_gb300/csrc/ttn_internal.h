@@ -118,6 +118,7 @@ void launch_hh_finish(const HhDesc* d, int ninst, int64_t mnmax, cudaStream_t s)
 void launch_hh_tall(const HhDesc* d, int ninst, cudaStream_t s);
 // CTAs that the cooperative panel kernel may use (all co-resident on the device)
 int hh_coop_capacity();
+int hh_coop_rows();  // rows of one of its CTAs in one pass
 // one panel [p0, p0 + HH_B) of every instance in one cooperative launch of nctas CTAs
 // (instance i owns CTAs [cta0, cta0 + ncta)); grid-wide waits are bounded and set *err
 void launch_hh_panel_coop(const HhDesc* d, int ninst, int nctas, int p0, int* err,
