@@ -29,6 +29,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "tn_internal.h"
 
 namespace tn {
@@ -110,28 +112,25 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 }
 
 // K-major SWIZZLE_128B shared-memory matrix descriptor (start address, LBO = 16 B,
-// SBO = 1024 B between 8-row groups, descriptor version 1, layout type 2 = 128B swizzle).
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= uint64_t((saddr & 0x3FFFF) >> 4);
-    d |= uint64_t(1) << 16;
-    d |= uint64_t(1024 >> 4) << 32;
-    d |= uint64_t(1) << 46;
-    d |= uint64_t(2) << 61;
-    return d;
+// SBO = 1024 B between 8-row groups, descriptor version 1, layout type 2 = 128B swizzle):
+// low and high 32 bits; the start address, in 16-byte units, is the low word's lower half
+__device__ __forceinline__ uint32_t sdesc_lo(uint32_t saddr) {
+    return ((saddr & 0x3FFFF) >> 4) | (1u << 16);
 }
+constexpr uint32_t SDESC_HI = (1024 >> 4) | (1u << 14) | (2u << 29);
 
 // Instruction descriptor of kind::f16: D = F32, A = B = BF16, both K-major, N = 64, M = 128.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
-                                         uint32_t accumulate) {
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo,
+                                         uint32_t idesc, bool accumulate) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+        "{\n .reg .pred p;\n .reg .b64 a, b;\n setp.ne.b32 p, %4, 0;\n"
+        " mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n" ::"r"(tmem_d),
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "r"(SDESC_HI));
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -383,12 +382,17 @@ struct __align__(8) SplitShared {
     int err;
 };
 
+// SL slices per operand.  The issuing thread's code is unrolled over the slice pairs: computing
+// the pair, its level, its ring stages and descriptors in loops took it 380 clocks a pair, 5700 a
+// k tile, three times what the tensor core needs for 60 products of 128 x 64 x 16.
+template <int SL>
 __global__ void __launch_bounds__(THREADS, 1)
 split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
                   const SplitTask* __restrict__ tasks, const uint8_t* __restrict__ apack,
                   const uint8_t* __restrict__ bpack, const int* __restrict__ ea,
-                  const int* __restrict__ eb, const __grid_constant__ Bases b, int slices,
+                  const int* __restrict__ eb, const __grid_constant__ Bases b,
                   int* __restrict__ err) {
+    constexpr int slices = SL;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // 1024-byte aligned stage ring (the swizzle atom needs it)
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -462,6 +466,7 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
+            const uint32_t ring_lo = sdesc_lo(smem_u32(ring));
             uint32_t g = 0;       // stage counter (matches the producer)
             uint32_t chunk = 0;   // accumulation chunk counter (TMEM double buffer)
             for (int it = blockIdx.x; it < nitems && !*serr; it += gridDim.x) {
@@ -473,38 +478,43 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
                     const int buf = chunk & 1;
                     if (!mbar_wait(&sh->tempty[buf], ((chunk >> 1) & 1) ^ 1, err, serr)) break;
                     asm volatile("tcgen05.fence::after_thread_sync;");
-                    uint32_t started = 0;  // accumulators written in this chunk
                     const int k1 = min(k0 + KC, tk.nkt);
                     bool ok = true;
                     for (int kt = k0; kt < k1 && ok; ++kt) {
                         const uint32_t g0 = g;
                         // 16-deep steps with valid k (the others would add zeros)
                         const int nkk = split_ksteps(tk.kmask, kt);
-                        for (int t = 0; t < slices; ++t) {
-                            const uint32_t gg = g0 + t;
-                            if (!mbar_wait(&sh->full[gg % NST], (gg / NST) & 1, err, serr)) {
+                        const bool fresh = kt == k0;  // the accumulators start anew
+                        uint32_t ad[SL], bd[SL];      // descriptors of the slices' tiles
+#pragma unroll
+                        for (int t = 0; t < SL; ++t) {
+                            const uint32_t st = (g0 + t) % NST;
+                            if (!mbar_wait(&sh->full[st], ((g0 + t) / NST) & 1, err, serr)) {
                                 ok = false;
                                 break;
                             }
                             asm volatile("tcgen05.fence::after_thread_sync;");
-                            // pairs (i, j) with max(i, j) == t and i + j <= slices - 1
-                            // (0-based slices: level = i + j + 2)
+                            ad[t] = ring_lo + st * (STAGE >> 4);
+                            bd[t] = ad[t] + (A_TILE >> 4);
+                            // pairs (i, t) and (t, i) with i + t <= slices - 1 (0-based
+                            // slices: level = i + t + 2, the fourth accumulator from 5 on); the
+                            // first of their accumulators are (0, 0), (0, 1), (1, 1) and (1, 2)
+#pragma unroll
                             for (int i = 0; i <= t; ++i) {
-                                for (int jj = 0; jj < 2; ++jj) {
-                                    const int j = jj == 0 ? t : i;
-                                    const int ii = jj == 0 ? i : t;
-                                    if (jj == 1 && i == t) continue;  // (t, t) once
-                                    if (ii + j > slices - 1) continue;
-                                    const int lvl = min(ii + j, NACC - 1);
-                                    const uint32_t sa = smem_u32(ring + ((g0 + ii) % NST) * STAGE);
-                                    const uint32_t sb = smem_u32(ring + ((g0 + j) % NST) * STAGE + A_TILE);
-                                    const uint32_t td = tmem + uint32_t(buf * NACC * BN + lvl * BN);
-                                    for (int kk = 0; kk < nkk; ++kk) {
-                                        mma_bf16(td, sdesc(sa + kk * 32), sdesc(sb + kk * 32), idesc,
-                                                 (started >> lvl) & 1);
-                                        started |= 1u << lvl;
-                                    }
-                                }
+                                if (i + t > SL - 1) continue;
+                                const int lvl = i + t < NACC - 1 ? i + t : NACC - 1;
+                                const uint32_t td = tmem + uint32_t(buf * NACC * BN + lvl * BN);
+                                const bool first = t < 2 || (i == 1 && t == 2);
+#pragma unroll
+                                for (int kk = 0; kk < BKT / 16; ++kk)
+                                    if (kk < nkk)
+                                        mma_bf16(td, ad[i] + 2 * kk, bd[t] + 2 * kk, idesc,
+                                                 !(first && kk == 0 && fresh));
+                                if (i == t) continue;
+#pragma unroll
+                                for (int kk = 0; kk < BKT / 16; ++kk)
+                                    if (kk < nkk)
+                                        mma_bf16(td, ad[t] + 2 * kk, bd[i] + 2 * kk, idesc, true);
                             }
                         }
                         if (!ok) break;
@@ -568,17 +578,21 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
             if (!ok) break;
             if (ncol == 0) continue;
             double* C = b.p[tk.cbuf] + tk.coff + gr + int64_t(item.nt * BN) * tk.ldc;
+            // (left at the block's last column: the code of the 32 columns is long, and stepping
+            // over unused ones costs an instruction fetch each)
 #pragma unroll
-            for (int c = 0; c < HC; ++c) {
-                const int tc = c % 16 + 16 * h + 32 * (c / 16);
-                if (tc >= ncol) continue;
-                const int e = er + __shfl_sync(0xffffffffu, ec, c) - 16;
-                const double v = scale2(widen(hi[c]) + widen(lo[c]), e);
-                if (gr < tk.m) {
-                    double* out = C + int64_t(tc) * tk.ldc;
-                    *out = tk.accum ? *out + v : v;
+            for (int g = 0; g < 2; ++g)
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const int c = 16 * g + k, tc = k + 16 * h + 32 * g;
+                    if (tc >= ncol) break;
+                    const int e = er + __shfl_sync(0xffffffffu, ec, c) - 16;
+                    const double v = scale2(widen(hi[c]) + widen(lo[c]), e);
+                    if (gr < tk.m) {
+                        double* out = C + int64_t(tc) * tk.ldc;
+                        *out = tk.accum ? *out + v : v;
+                    }
                 }
-            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -627,15 +641,17 @@ void launch_split_gemm(const SplitItem* items, int nitems, const SplitTask* task
     if (nitems <= 0) return;
     TN_REQUIRE(slices >= 4 && slices <= 7, "split precision needs 4..7 slices");
     const size_t shm = size_t(NST) * STAGE + sizeof(SplitShared) + 1024;
-    static bool attr = false;
-    if (!attr) {
-        TN_CUDA(cudaFuncSetAttribute(split_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(shm)));
-        attr = true;
+    auto* kernel = slices == 4   ? split_gemm_kernel<4>
+                   : slices == 5 ? split_gemm_kernel<5>
+                   : slices == 6 ? split_gemm_kernel<6>
+                                 : split_gemm_kernel<7>;
+    static std::atomic<bool> attr[8];
+    if (!attr[slices]) {
+        TN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
+        attr[slices] = true;
     }
     const int grid = nitems < nsm ? nitems : nsm;
-    split_gemm_kernel<<<grid, THREADS, shm, s>>>(items, nitems, tasks, apack, bpack, ea, eb, b,
-                                                  slices, err);
+    kernel<<<grid, THREADS, shm, s>>>(items, nitems, tasks, apack, bpack, ea, eb, b, err);
     TN_CUDA(cudaGetLastError());
     count_launch();
 }
