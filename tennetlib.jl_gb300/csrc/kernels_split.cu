@@ -85,6 +85,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
     }
 }
 
+// the error flag as the whole warp sees it (lanes may read it at different times)
+__device__ __forceinline__ bool warp_err(volatile int* shared_err) {
+    return __any_sync(0xffffffffu, *shared_err != 0);
+}
+
 // Bounded wait used only to drain before exit (no error bookkeeping).
 __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
     const long long t0 = clock64();
@@ -96,18 +101,37 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-                 "r"(bytes)
-                 : "memory");
+// The whole warp runs the issuing code on values that are uniform to the compiler, with one
+// lane's predicate on the instructions: descriptors then live in uniform registers.  Issued from a
+// one-lane branch with per-thread values, each product took 230 clocks whatever its width
+// (measured alone: 71 from a branch, 39 for 16 columns, 48 for 64 and 64 for 128 this way), and a
+// k tile of one 16-deep step 5700 clocks instead of 2100.
+__device__ __forceinline__ uint32_t elect_lane() {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(r));
+    return r;
+}
+
+// (the copies of a stage, like the products, are issued by a whole warp with one lane's predicate)
+// a value that all lanes have alike, known as such to the compiler
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes, uint32_t lead) {
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n"
+        " @q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}\n" ::"r"(smem_u32(bar)),
+        "r"(bytes), "r"(lead)
+        : "memory");
 }
 
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes,
-                                         uint64_t* bar) {
+                                         uint64_t* bar, uint32_t lead) {
     asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-            "r"(smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
+        "{\n .reg .pred q;\n setp.ne.b32 q, %4, 0;\n"
+        " @q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+        "}\n" ::"r"(smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(bar)), "r"(lead)
         : "memory");
 }
 
@@ -125,18 +149,20 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo,
-                                         uint32_t idesc, bool accumulate) {
+                                         uint32_t idesc, bool accumulate, uint32_t lead) {
     asm volatile(
-        "{\n .reg .pred p;\n .reg .b64 a, b;\n setp.ne.b32 p, %4, 0;\n"
+        "{\n .reg .pred p, q;\n .reg .b64 a, b;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %6, 0;\n"
         " mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n" ::"r"(tmem_d),
-        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "r"(SDESC_HI));
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n" ::"r"(tmem_d),
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "r"(SDESC_HI), "r"(lead));
 }
 
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+__device__ __forceinline__ void mma_commit(uint64_t* bar, uint32_t lead) {
     asm volatile(
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            smem_u32(bar))
+        "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(
+            smem_u32(bar)),
+        "r"(lead)
         : "memory");
 }
 
@@ -382,7 +408,7 @@ struct __align__(8) SplitShared {
     int err;
 };
 
-// SL slices per operand.  The issuing thread's code is unrolled over the slice pairs: computing
+// SL slices per operand.  The issuing code is unrolled over the slice pairs: computing
 // the pair, its level, its ring stages and descriptors in loops took it 380 clocks a pair, 5700 a
 // k tile, three times what the tensor core needs for 60 products of 128 x 64 x 16.
 template <int SL>
@@ -430,66 +456,75 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
 
     if (warp == 0) {
         // ---------------- producer ----------------
-        if (lane == 0) {
-            // test hook (tn_ctx_inject_wait_timeout, code 1): CTA 0 withholds the copies of its
-            // first stage, so that the MMA warp's wait on it runs out and every role drains
-            const bool withhold = blockIdx.x == 0 && atomicCAS(err + 1, 1, 0) == 1;
-            uint32_t g = 0;  // global stage counter
-            for (int it = blockIdx.x; it < nitems && !*serr; it += gridDim.x) {
-                const SplitItem item = it == int(blockIdx.x) ? item0 : items[it];
-                const SplitTask tk = it == int(blockIdx.x) ? task0 : tasks[item.task];
-                // the 8-row atoms that hold rows of the block (the rest of the stage keeps
-                // what was there: it only reaches outputs that are not stored)
-                const uint32_t abytes = uint32_t(min(BM, tk.m - item.mt * BM) + 7) / 8 * 1024;
-                const uint32_t bbytes = uint32_t(min(BN, tk.n - item.nt * BN) + 7) / 8 * 1024;
-                for (int kt = 0; kt < tk.nkt && !*serr; ++kt)
-                    for (int t = 0; t < slices; ++t, ++g) {
-                        const int st = g % NST;
-                        const uint32_t ph = (g / NST) & 1;
-                        if (!mbar_wait(&sh->empty[st], ph ^ 1, err, serr)) break;
-                        if (withhold && g == 0) continue;
-                        uint8_t* dst = ring + st * STAGE;
-                        mbar_expect_tx(&sh->full[st], abytes + bbytes);
-                        const int64_t ao = tk.a_off + (int64_t(item.mt) * tk.nkt + kt) * slices * A_TILE +
-                                           int64_t(t) * A_TILE;
-                        const int64_t bo = tk.b_off + (int64_t(item.nt) * tk.nkt + kt) * slices * B_TILE +
-                                           int64_t(t) * B_TILE;
-                        bulk_g2s(dst, apack + ao, abytes, &sh->full[st]);
-                        bulk_g2s(dst + A_TILE, bpack + bo, bbytes, &sh->full[st]);
-                    }
-            }
-            // before the CTA may exit, every copy this thread issued must have landed (in the
-            // normal path the MMA warp has consumed them all; after an error this drains)
-            for (uint32_t gg = (g > NST ? g - NST : 0); gg < g; ++gg)
-                mbar_drain(&sh->full[gg % NST], (gg / NST) & 1);
+        const uint32_t lead = elect_lane();
+        // test hook (tn_ctx_inject_wait_timeout, code 1): CTA 0 withholds the copies of its
+        // first stage, so that the MMA warp's wait on it runs out and every role drains
+        bool withhold = false;
+        if (blockIdx.x == 0) withhold = __any_sync(0xffffffffu, lead && atomicCAS(err + 1, 1, 0) == 1);
+        uint32_t g = 0;  // global stage counter
+        for (int it = blockIdx.x; it < nitems && !warp_err(serr); it += gridDim.x) {
+            const SplitItem item = it == int(blockIdx.x) ? item0 : items[it];
+            const SplitTask tk = it == int(blockIdx.x) ? task0 : tasks[item.task];
+            // the 8-row atoms that hold rows of the block (the rest of the stage keeps
+            // what was there: it only reaches outputs that are not stored)
+            const uint32_t abytes = uniform(uint32_t(min(BM, tk.m - item.mt * BM) + 7) / 8 * 1024);
+            const uint32_t bbytes = uniform(uint32_t(min(BN, tk.n - item.nt * BN) + 7) / 8 * 1024);
+            const int nkt = int(uniform(uint32_t(tk.nkt)));
+            const uint8_t* asrc = apack + tk.a_off + int64_t(item.mt) * tk.nkt * slices * A_TILE;
+            const uint8_t* bsrc = bpack + tk.b_off + int64_t(item.nt) * tk.nkt * slices * B_TILE;
+            bool ok = true;
+            for (int kt = 0; kt < nkt && ok; ++kt)
+                for (int t = 0; t < slices; ++t, ++g, asrc += A_TILE, bsrc += B_TILE) {
+                    const int st = g % NST;
+                    const uint32_t ph = (g / NST) & 1;
+                    ok = __all_sync(0xffffffffu, mbar_wait(&sh->empty[st], ph ^ 1, err, serr));
+                    if (!ok) break;
+                    if (withhold && g == 0) continue;
+                    uint8_t* dst = ring + st * STAGE;
+                    mbar_expect_tx(&sh->full[st], abytes + bbytes, lead);
+                    bulk_g2s(dst, asrc, abytes, &sh->full[st], lead);
+                    bulk_g2s(dst + A_TILE, bsrc, bbytes, &sh->full[st], lead);
+                }
         }
+        // before the CTA may exit, every copy this warp issued must have landed (in the normal
+        // path the MMA warp has consumed them all; after an error this drains)
+        for (uint32_t gg = (g > NST ? g - NST : 0); gg < g; ++gg)
+            mbar_drain(&sh->full[gg % NST], (gg / NST) & 1);
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t ring_lo = sdesc_lo(smem_u32(ring));
+        {
+            const uint32_t lead = elect_lane();
+            const uint32_t ring_lo = uniform(sdesc_lo(smem_u32(ring)));
+            const uint32_t tmem_u = uniform(tmem);
             uint32_t g = 0;       // stage counter (matches the producer)
             uint32_t chunk = 0;   // accumulation chunk counter (TMEM double buffer)
-            for (int it = blockIdx.x; it < nitems && !*serr; it += gridDim.x) {
+            for (int it = blockIdx.x; it < nitems && !warp_err(serr); it += gridDim.x) {
                 const SplitItem item = it == int(blockIdx.x) ? item0 : items[it];
                 const SplitTask tk = it == int(blockIdx.x) ? task0 : tasks[item.task];
                 // N covers the block's columns (a multiple of 16)
-                const uint32_t idesc = idesc_bf16(BM, (min(BN, tk.n - item.nt * BN) + 15) / 16 * 16);
-                for (int k0 = 0; k0 < tk.nkt && !*serr; k0 += KC, ++chunk) {
+                const uint32_t idesc =
+                    uniform(idesc_bf16(BM, (min(BN, tk.n - item.nt * BN) + 15) / 16 * 16));
+                const int nkt = int(uniform(uint32_t(tk.nkt)));
+                const uint64_t kmask = uint64_t(uniform(uint32_t(tk.kmask >> 32))) << 32 |
+                                       uniform(uint32_t(tk.kmask));
+                for (int k0 = 0; k0 < nkt && !warp_err(serr); k0 += KC, ++chunk) {
                     const int buf = chunk & 1;
-                    if (!mbar_wait(&sh->tempty[buf], ((chunk >> 1) & 1) ^ 1, err, serr)) break;
+                    if (!__all_sync(0xffffffffu, mbar_wait(&sh->tempty[buf], ((chunk >> 1) & 1) ^ 1, err, serr)))
+                        break;
                     asm volatile("tcgen05.fence::after_thread_sync;");
-                    const int k1 = min(k0 + KC, tk.nkt);
+                    const int k1 = min(k0 + KC, nkt);
                     bool ok = true;
                     for (int kt = k0; kt < k1 && ok; ++kt) {
                         const uint32_t g0 = g;
                         // 16-deep steps with valid k (the others would add zeros)
-                        const int nkk = split_ksteps(tk.kmask, kt);
+                        const int nkk = split_ksteps(kmask, kt);
                         const bool fresh = kt == k0;  // the accumulators start anew
                         uint32_t ad[SL], bd[SL];      // descriptors of the slices' tiles
 #pragma unroll
                         for (int t = 0; t < SL; ++t) {
                             const uint32_t st = (g0 + t) % NST;
-                            if (!mbar_wait(&sh->full[st], ((g0 + t) / NST) & 1, err, serr)) {
+                            if (!__all_sync(0xffffffffu,
+                                            mbar_wait(&sh->full[st], ((g0 + t) / NST) & 1, err, serr))) {
                                 ok = false;
                                 break;
                             }
@@ -503,32 +538,30 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
                             for (int i = 0; i <= t; ++i) {
                                 if (i + t > SL - 1) continue;
                                 const int lvl = i + t < NACC - 1 ? i + t : NACC - 1;
-                                const uint32_t td = tmem + uint32_t(buf * NACC * BN + lvl * BN);
+                                const uint32_t td = tmem_u + uint32_t(buf * NACC * BN + lvl * BN);
                                 const bool first = t < 2 || (i == 1 && t == 2);
-#pragma unroll
-                                for (int kk = 0; kk < BKT / 16; ++kk)
-                                    if (kk < nkk)
-                                        mma_bf16(td, ad[i] + 2 * kk, bd[t] + 2 * kk, idesc,
-                                                 !(first && kk == 0 && fresh));
+#pragma unroll 1
+                                for (int kk = 0; kk < nkk; ++kk)
+                                    mma_bf16(td, ad[i] + 2 * kk, bd[t] + 2 * kk, idesc,
+                                             !(first && kk == 0 && fresh), lead);
                                 if (i == t) continue;
-#pragma unroll
-                                for (int kk = 0; kk < BKT / 16; ++kk)
-                                    if (kk < nkk)
-                                        mma_bf16(td, ad[t] + 2 * kk, bd[i] + 2 * kk, idesc, true);
+#pragma unroll 1
+                                for (int kk = 0; kk < nkk; ++kk)
+                                    mma_bf16(td, ad[t] + 2 * kk, bd[i] + 2 * kk, idesc, true, lead);
                             }
                         }
                         if (!ok) break;
-                        for (int t = 0; t < slices; ++t) mma_commit(&sh->empty[(g0 + t) % NST]);
+                        for (int t = 0; t < slices; ++t) mma_commit(&sh->empty[(g0 + t) % NST], lead);
                         g = g0 + slices;
                     }
                     if (!ok) break;
                     // with slices >= 4 every k tile writes all four levels, so every
                     // accumulator of this chunk has been (re)initialised
-                    mma_commit(&sh->tfull[buf]);
+                    mma_commit(&sh->tfull[buf], lead);
                 }
             }
-            // every MMA this thread issued completes before TMEM is released
-            mma_commit(&sh->done);
+            // every MMA this warp issued completes before TMEM is released
+            mma_commit(&sh->done, lead);
             mbar_drain(&sh->done, 0);
         }
     } else {
