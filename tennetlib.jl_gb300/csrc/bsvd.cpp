@@ -53,19 +53,20 @@ struct GemmRun {
         flops += g.flops;
         cudaStream_t st = ctx->stream;
         if (!split || force_fp64) {
-            g.finalize(st);
             launch_gemm_f64(g, bs, st);
             return;
         }
         auto sp = make_split_plan(g, SVD_SLICES, st, true);
-        launch_split_pack(sp->dajobs.as<PackJob>(), (int)sp->ajobs.size(), sp->daks.as<KTileSrc>(),
-                          bs, sp->ap, sp->eap, sp->slices, split_tile_rows_a(), st, sp->a_maxnkt,
+        launch_split_pack(sp->tab.at<PackJob>(sp->oajobs), (int)sp->ajobs.size(),
+                          sp->tab.at<KTileSrc>(sp->oaks), bs, sp->ap, sp->eap, sp->slices,
+                          split_tile_rows_a(), st, sp->a_maxnkt,
                           sp->amax.as<unsigned long long>(), sp->ea_n);
-        launch_split_pack(sp->dbjobs.as<PackJob>(), (int)sp->bjobs.size(), sp->dbks.as<KTileSrc>(),
-                          bs, sp->bp, sp->ebp, sp->slices, split_tile_rows_b(), st, sp->b_maxnkt,
+        launch_split_pack(sp->tab.at<PackJob>(sp->objobs), (int)sp->bjobs.size(),
+                          sp->tab.at<KTileSrc>(sp->obks), bs, sp->bp, sp->ebp, sp->slices,
+                          split_tile_rows_b(), st, sp->b_maxnkt,
                           sp->bmax.as<unsigned long long>(), sp->eb_n);
-        launch_split_gemm(sp->ditems.as<SplitItem>(), (int)sp->items.size(),
-                          sp->dtasks.as<SplitTask>(), sp->ap, sp->bp, sp->eap, sp->ebp, bs,
+        launch_split_gemm(sp->tab.at<SplitItem>(sp->oitems), (int)sp->items.size(),
+                          sp->tab.at<SplitTask>(sp->otasks), sp->ap, sp->bp, sp->eap, sp->ebp, bs,
                           sp->slices, ctx->err.as<int>(), ctx->nsm, st);
     }
 };

@@ -195,13 +195,6 @@ bool need_right(const tn_mpo* H, int site, int c, int s) {
 // -------------------------------------------------------------------------------------
 // split-precision GEMM plans
 // -------------------------------------------------------------------------------------
-template <class T>
-void upload_vec(DevBuf& b, const std::vector<T>& v, cudaStream_t s) {
-    b.alloc(std::max<size_t>(v.size() * sizeof(T), 16), s);
-    if (!v.empty())
-        TN_CUDA(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
-}
-
 std::unique_ptr<SplitPlan> make_split(const GemmPlan& g, int slices, bool a_static,
                                       bool b_static, cudaStream_t st, bool own_packs = true) {
     for (const Seg& sg : g.segs)
@@ -314,47 +307,48 @@ std::unique_ptr<SplitPlan> make_split(const GemmPlan& g, int slices, bool a_stat
     sp->eb_n = ebo;
     for (const auto& j : sp->ajobs) sp->a_maxnkt = std::max(sp->a_maxnkt, j.nkt);
     for (const auto& j : sp->bjobs) sp->b_maxnkt = std::max(sp->b_maxnkt, j.nkt);
-    sp->amax.alloc(size_t(std::max<int64_t>(eao, 1)) * 8, st);
-    sp->bmax.alloc(size_t(std::max<int64_t>(ebo, 1)) * 8, st);
-    upload_vec(sp->dtasks, sp->tasks, st);
-    upload_vec(sp->ditems, sp->items, st);
-    upload_vec(sp->dajobs, sp->ajobs, st);
-    upload_vec(sp->dbjobs, sp->bjobs, st);
-    upload_vec(sp->daks, sp->aks, st);
-    upload_vec(sp->dbks, sp->bks, st);
-    if (own_packs) {
-        sp->apack.alloc(size_t(std::max<int64_t>(aoff, 1024)), st);
-        sp->bpack.alloc(size_t(std::max<int64_t>(boff, 1024)), st);
-        sp->ea.alloc(size_t(std::max<int64_t>(eao, 4)) * 4, st);
-        sp->eb.alloc(size_t(std::max<int64_t>(ebo, 4)) * 4, st);
-        sp->ap = sp->apack.as<uint8_t>();
-        sp->bp = sp->bpack.as<uint8_t>();
-        sp->eap = sp->ea.as<int>();
-        sp->ebp = sp->eb.as<int>();
+    if (split_pack_needs_max(sp->a_maxnkt)) sp->amax.alloc(size_t(std::max<int64_t>(eao, 1)) * 8, st);
+    if (split_pack_needs_max(sp->b_maxnkt)) sp->bmax.alloc(size_t(std::max<int64_t>(ebo, 1)) * 8, st);
+    sp->otasks = sp->tab.add(sp->tasks);
+    sp->oitems = sp->tab.add(sp->items);
+    sp->oajobs = sp->tab.add(sp->ajobs);
+    sp->objobs = sp->tab.add(sp->bjobs);
+    sp->oaks = sp->tab.add(sp->aks);
+    sp->obks = sp->tab.add(sp->bks);
+    sp->tab.upload(st);
+    if (own_packs) {  // (aoff and boff are multiples of 1024)
+        sp->packs.alloc(size_t(aoff + boff + 4 * (eao + ebo) + 1024), st);
+        sp->ap = sp->packs.as<uint8_t>();
+        sp->bp = sp->ap + aoff;
+        sp->eap = reinterpret_cast<int*>(sp->bp + boff);
+        sp->ebp = sp->eap + eao;
     }
     return sp;
 }
 
 // pack the operands that need it, then run the tensor-core GEMM; times packs and MMA
-void run_split(tn_ctx* ctx, SplitPlan& sp, const Bases& bs, int* mma_ev0, int* mma_ev1) {
+void run_split(tn_ctx* ctx, SplitPlan& sp, const Bases& bs, int* mma_ev0, int* mma_ev1,
+               int start = -1) {
     cudaStream_t st = ctx->stream;
-    const int p0 = ctx->timer.mark();
+    const int p0 = start >= 0 ? start : ctx->timer.mark();  // start: a mark made just now
     if (!sp.a_static || !sp.a_packed) {
-        launch_split_pack(sp.dajobs.as<PackJob>(), (int)sp.ajobs.size(), sp.daks.as<KTileSrc>(), bs,
+        launch_split_pack(sp.tab.at<PackJob>(sp.oajobs), (int)sp.ajobs.size(),
+                          sp.tab.at<KTileSrc>(sp.oaks), bs,
                           sp.ap, sp.eap, sp.slices, split_tile_rows_a(), st, sp.a_maxnkt,
                           sp.amax.as<unsigned long long>(), sp.ea_n);
         sp.a_packed = true;
     }
     if (!sp.b_static || !sp.b_packed) {
-        launch_split_pack(sp.dbjobs.as<PackJob>(), (int)sp.bjobs.size(), sp.dbks.as<KTileSrc>(), bs,
+        launch_split_pack(sp.tab.at<PackJob>(sp.objobs), (int)sp.bjobs.size(),
+                          sp.tab.at<KTileSrc>(sp.obks), bs,
                           sp.bp, sp.ebp, sp.slices, split_tile_rows_b(), st, sp.b_maxnkt,
                           sp.bmax.as<unsigned long long>(), sp.eb_n);
         sp.b_packed = true;
     }
     const int p1 = ctx->timer.mark();
     ctx->timer.add(T_PACK, p0, p1);
-    launch_split_gemm(sp.ditems.as<SplitItem>(), (int)sp.items.size(), sp.dtasks.as<SplitTask>(),
-                      sp.ap, sp.bp, sp.eap, sp.ebp, bs, sp.slices, ctx->err.as<int>(), ctx->nsm, st);
+    launch_split_gemm(sp.tab.at<SplitItem>(sp.oitems), (int)sp.items.size(),
+                      sp.tab.at<SplitTask>(sp.otasks), sp.ap, sp.bp, sp.eap, sp.ebp, bs, sp.slices, ctx->err.as<int>(), ctx->nsm, st);
     const int p2 = ctx->timer.mark();
     if (mma_ev0) *mma_ev0 = p1;
     if (mma_ev1) *mma_ev1 = p2;
@@ -479,8 +473,6 @@ void env_left_step(tn_env* env, int i) {
         set_im(bs, S_Y, Lout.lay.size);
         GemmPlan c1 = complex_plan(g1, 0), c3 = complex_plan(g3, 1u << S_X);
         CombPlan cc = complex_comb(cb);
-        c1.finalize(st);
-        c3.finalize(st);
         cc.finalize(st);
         launch_gemm_f64(c1, bs, st);
         launch_combine(cc, bs, st);
@@ -488,8 +480,6 @@ void env_left_step(tn_env* env, int i) {
         launch_scale_into(Lout.buf.d() + 2 * Lout.lay.size, Lout.buf.d() + Lout.lay.size,
                           nullptr, -1.0, Lout.lay.size, st);
     } else {
-        g1.finalize(st);
-        g3.finalize(st);
         cb.finalize(st);
         run_gemm(ctx, g1, bs);
         launch_combine(cb, bs, st);
@@ -594,8 +584,6 @@ void env_right_step(tn_env* env, int i) {
         set_im(bs, S_Y, Rout.lay.size);
         GemmPlan c1 = complex_plan(g1, 0), c3 = complex_plan(g3, 1u << S_X);
         CombPlan cc = complex_comb(cb);
-        c1.finalize(st);
-        c3.finalize(st);
         cc.finalize(st);
         launch_gemm_f64(c1, bs, st);
         launch_combine(cc, bs, st);
@@ -603,8 +591,6 @@ void env_right_step(tn_env* env, int i) {
         launch_scale_into(Rout.buf.d() + 2 * Rout.lay.size, Rout.buf.d() + Rout.lay.size,
                           nullptr, -1.0, Rout.lay.size, st);
     } else {
-        g1.finalize(st);
-        g3.finalize(st);
         cb.finalize(st);
         run_gemm(ctx, g1, bs);
         launch_combine(cb, bs, st);
@@ -748,8 +734,6 @@ std::unique_ptr<Heff2Plan> build_heff2(tn_env* env, int p) {
                 P->g3.add_seg(S_T2, sg.zo, ph.rows[mo], 0, S_R, sg.ro, sg.Drp, 1, sg.Dr);
         }
     cudaStream_t st = env->ctx->stream;
-    P->g1.finalize(st);
-    P->g3.finalize(st);
     P->cb.finalize(st);
     P->ysize = y;
     P->zsize = z;
@@ -759,8 +743,6 @@ std::unique_ptr<Heff2Plan> build_heff2(tn_env* env, int p) {
         P->g1c = complex_plan(P->g1, 0);
         P->g3c = complex_plan(P->g3, 0);
         P->cbc = complex_comb(P->cb);
-        P->g1c.finalize(st);
-        P->g3c.finalize(st);
         P->cbc.finalize(st);
         P->flops = P->g1c.flops + P->g3c.flops + P->cbc.flops;
     }
@@ -810,7 +792,7 @@ void heff_apply(tn_env* env, Heff2Plan& P, const double* x, double* y) {
                 P.s3c = make_split(*u3, ctx->slices, false, true, ctx->stream);   // B = R
             }
             int a0 = -1, a1 = -1, b0 = -1, b1 = -1;
-            run_split(ctx, *P.s1c, bs, &a0, &a1);
+            run_split(ctx, *P.s1c, bs, &a0, &a1, e0);
             launch_combine(P.cbc, bs, ctx->stream);
             run_split(ctx, *P.s3c, bs, &b0, &b1);
             ctx->timer.add(T_GEMM, a0, a1);
@@ -824,7 +806,7 @@ void heff_apply(tn_env* env, Heff2Plan& P, const double* x, double* y) {
         env->matvecs++;
         env->heff_flops += P.flops;
         env->gemm_flops += P.g1c.flops + P.g3c.flops;
-        env->gemm_launches += (P.g1c.tiles.empty() ? 0 : 1) + (P.g3c.tiles.empty() ? 0 : 1);
+        env->gemm_launches += (P.g1c.tasks.empty() ? 0 : 1) + (P.g3c.tasks.empty() ? 0 : 1);
         return;
     }
     if (ctx->prec == TN_PREC_SPLIT) {
@@ -851,7 +833,7 @@ void heff_apply(tn_env* env, Heff2Plan& P, const double* x, double* y) {
     env->matvecs++;
     env->heff_flops += P.flops;
     env->gemm_flops += P.g1.flops + P.g3.flops;
-    env->gemm_launches += (P.g1.tiles.empty() ? 0 : 1) + (P.g3.tiles.empty() ? 0 : 1);
+    env->gemm_launches += (P.g1.tasks.empty() ? 0 : 1) + (P.g3.tasks.empty() ? 0 : 1);
 }
 
 // -------------------------------------------------------------------------------------
@@ -939,8 +921,6 @@ std::unique_ptr<Heff1Plan> build_heff1(tn_env* env, int p) {
                 P->g3.add_seg(S_T2, sg.zo, Dlp, 0, S_R, sg.ro, sg.Drp, 1, sg.Dr);
         }
     cudaStream_t st = env->ctx->stream;
-    P->g1.finalize(st);
-    P->g3.finalize(st);
     P->cb.finalize(st);
     P->ysize = y;
     P->zsize = z;
@@ -949,8 +929,6 @@ std::unique_ptr<Heff1Plan> build_heff1(tn_env* env, int p) {
         P->g1c = complex_plan(P->g1, 0);
         P->g3c = complex_plan(P->g3, 0);
         P->cbc = complex_comb(P->cb);
-        P->g1c.finalize(st);
-        P->g3c.finalize(st);
         P->cbc.finalize(st);
         P->flops = P->g1c.flops + P->g3c.flops + P->cbc.flops;
     }
@@ -1000,7 +978,7 @@ void heff1_apply(tn_env* env, Heff1Plan& P, const double* x, double* y) {
                 P.s3c = make_split(*u3, ctx->slices, false, true, ctx->stream);   // B = R
             }
             int a0 = -1, a1 = -1, b0 = -1, b1 = -1;
-            run_split(ctx, *P.s1c, bs, &a0, &a1);
+            run_split(ctx, *P.s1c, bs, &a0, &a1, e0);
             launch_combine(P.cbc, bs, ctx->stream);
             run_split(ctx, *P.s3c, bs, &b0, &b1);
             ctx->timer.add(T_GEMM, a0, a1);
@@ -1014,7 +992,7 @@ void heff1_apply(tn_env* env, Heff1Plan& P, const double* x, double* y) {
         env->matvecs++;
         env->heff_flops += P.flops;
         env->gemm_flops += P.g1c.flops + P.g3c.flops;
-        env->gemm_launches += (P.g1c.tiles.empty() ? 0 : 1) + (P.g3c.tiles.empty() ? 0 : 1);
+        env->gemm_launches += (P.g1c.tasks.empty() ? 0 : 1) + (P.g3c.tasks.empty() ? 0 : 1);
         return;
     }
     if (ctx->prec == TN_PREC_SPLIT) {
@@ -1035,7 +1013,7 @@ void heff1_apply(tn_env* env, Heff1Plan& P, const double* x, double* y) {
     env->matvecs++;
     env->heff_flops += P.flops;
     env->gemm_flops += P.g1.flops + P.g3.flops;
-    env->gemm_launches += (P.g1.tiles.empty() ? 0 : 1) + (P.g3.tiles.empty() ? 0 : 1);
+    env->gemm_launches += (P.g1.tasks.empty() ? 0 : 1) + (P.g3.tasks.empty() ? 0 : 1);
 }
 
 // copy a site tensor between the left-grouped and right-grouped layouts (block copies)
@@ -1145,11 +1123,9 @@ void form_phi(tn_env* env, int p, const PhiLayout& ph, double* out) {
         set_im(bs, S_B, Y.lay.size);
         set_im(bs, S_Y, ph.size);
         GemmPlan c = complex_plan(g, 0);
-        c.finalize(env->ctx->stream);
         launch_gemm_f64(c, bs, env->ctx->stream);
         return;
     }
-    g.finalize(env->ctx->stream);
     launch_gemm_f64(g, bs, env->ctx->stream);
 }
 
@@ -2072,7 +2048,6 @@ void replace_bond_noise(tn_env* env, int p, Heff2Plan& P, const double* phi,
         tbuf.alloc(size_t(std::max<int64_t>(t, 1)) * 8, st);
         bs.p[S_T2] = tbuf.d();
         if (!gt.tasks.empty()) {
-            if (ctx->prec != TN_PREC_SPLIT) gt.finalize(st);
             run_gemm(ctx, gt, bs);
         }
         for (int k = 0; k < nm; ++k) {
@@ -2199,7 +2174,6 @@ void replace_bond_noise(tn_env* env, int p, Heff2Plan& P, const double* phi,
     tn_site& kept_site = left ? lsite : rsite;
     tn_site& other = left ? rsite : lsite;
     if (!g.tasks.empty()) {
-        g.finalize(st);
         Bases gb{};
         gb.p[S_X] = const_cast<double*>(phi);
         gb.p[S_A] = kept_site.buf.d();
@@ -2597,11 +2571,6 @@ void update_one_site(tn_env* env, int p, int ortho, const tn_update_params* prm,
         if (psi->cplx) {
             c1 = complex_plan(H0.g1, 0);
             c2 = complex_plan(H0.g2, 0);
-            c1.finalize(st);
-            c2.finalize(st);
-        } else {
-            H0.g1.finalize(st);
-            H0.g2.finalize(st);
         }
         env->cx.alloc(size_t(std::max<int64_t>(H0.tsize, 1)) * 8 * np, st);
         auto apply0 = [&](const double* x, double* y) {
@@ -2685,10 +2654,8 @@ void update_one_site(tn_env* env, int p, int ortho, const tn_update_params* prm,
             set_im(bs, S_A, nlay_old.size);
             set_im(bs, S_Y, nnew.lay.size);
             gc = complex_plan(g, 0);
-            gc.finalize(st);
             launch_gemm_f64(gc, bs, st);
         } else {
-            g.finalize(st);
             launch_gemm_f64(g, bs, st);  // the small bond matrix is multiplied in FP64
         }
         ctx->timer.add(T_SVD, e1, ctx->timer.mark());

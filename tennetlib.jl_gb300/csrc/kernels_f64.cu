@@ -25,7 +25,7 @@ namespace tn {
 // and the next chunk's loads in flight during the products.  Each output is one chain of fused
 // multiply-adds in segment order.  On the 64 x 64 x 16 tiles of 256 threads that this replaced
 // a 4 x 4 x 4 block took 16 us of multiplications by zeros.
-// The tile is GemmPlan::finalize's choice.  Measured, whole calls in FP64: DMRG run of a
+// The tile is GemmPlan::prepare's choice.  Measured, whole calls in FP64: DMRG run of a
 // 12-site chain 118 -> 71 ms, sweep of a 20-site cylinder at chi = 160 236 -> 95 ms, TDVP of
 // a 12-site chain (complex) 209 -> 91 ms, sweep of a 16-site tree at chi = 16 75 -> 41 ms.
 // ------------------------------------------------------------------------------------
@@ -497,12 +497,14 @@ VecPtrs make_ptrs(const double* const* V, int K) {
 }  // namespace
 
 void launch_gemm_f64(const GemmPlan& p, const Bases& b, cudaStream_t s) {
-    if (p.tiles.empty()) return;
+    if (p.tasks.empty()) return;
+    p.prepare(s);
+    if (p.ntiles == 0) return;
     auto* kernel = p.tile_n == 32   ? gemm_f64_kernel<32, 32>
                    : p.tile_n == 16 ? gemm_f64_kernel<16, 16>
                                     : gemm_f64_kernel<16, 8>;
-    kernel<<<unsigned(p.tiles.size()), GEMM_THREADS, 0, s>>>(
-        p.dsegs.as<Seg>(), p.dtasks.as<Task>(), p.dtiles.as<Tile>(), b);
+    kernel<<<unsigned(p.ntiles), GEMM_THREADS, 0, s>>>(
+        p.tab.at<Seg>(p.osegs), p.tab.at<Task>(p.otasks), p.tab.at<Tile>(p.otiles), b);
     TN_CUDA(cudaGetLastError());
     count_launch();
 }
@@ -510,7 +512,7 @@ void launch_gemm_f64(const GemmPlan& p, const Bases& b, cudaStream_t s) {
 void launch_combine(const CombPlan& p, const Bases& b, cudaStream_t s) {
     if (p.tiles.empty()) return;
     combine_kernel<<<unsigned(p.tiles.size()), 256, 0, s>>>(
-        p.douts.as<CombOut>(), p.dterms.as<CombTerm>(), p.dtiles.as<CombTile>(), b);
+        p.tab.at<CombOut>(p.oouts), p.tab.at<CombTerm>(p.oterms), p.tab.at<CombTile>(p.otiles), b);
     TN_CUDA(cudaGetLastError());
     count_launch();
 }

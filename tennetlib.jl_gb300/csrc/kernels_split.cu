@@ -643,6 +643,8 @@ int split_tile_bytes_b() { return B_TILE; }
 int split_tile_rows_a() { return BM; }
 int split_tile_rows_b() { return BN; }
 int split_ktile() { return BKT; }
+constexpr int KPER = 2;  // k tiles per CTA of the k-split pack
+bool split_pack_needs_max(int max_nkt) { return max_nkt > 2 * KPER; }
 
 void launch_split_pack(const PackJob* jobs, int njobs, const KTileSrc* ksrc, const Bases& b,
                        uint8_t* out, int* expo, int slices, int tile_rows, cudaStream_t s,
@@ -650,8 +652,7 @@ void launch_split_pack(const PackJob* jobs, int njobs, const KTileSrc* ksrc, con
     if (njobs <= 0) return;
     TN_REQUIRE(slices >= 4 && slices <= 7, "split precision needs 4..7 slices");
     TN_REQUIRE(tile_rows <= BM, "pack tile taller than the A tile");
-    constexpr int KPER = 2;  // k tiles per CTA of the k-split pack
-    if (max_nkt <= 2 * KPER || !gmax) {
+    if (!split_pack_needs_max(max_nkt) || !gmax) {
         const dim3 g(njobs, (tile_rows + PACK_ROWS - 1) / PACK_ROWS);
         split_pack_kernel<<<g, PACK_THREADS, 0, s>>>(jobs, ksrc, b, out, expo, slices, tile_rows);
         TN_CUDA(cudaGetLastError());

@@ -210,16 +210,9 @@ void GemmPlan::add_seg(int abuf, int64_t aoff, int lda, int ta, int bbuf, int64_
     flops += 2.0 * double(t.m) * double(t.n) * double(k);
 }
 
-template <class T>
-static void upload(DevBuf& b, const std::vector<T>& v, cudaStream_t s) {
-    size_t nb = std::max<size_t>(v.size() * sizeof(T), 16);
-    b.alloc(nb, s);
-    if (!v.empty())
-        TN_CUDA(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
-}
-
-void GemmPlan::finalize(cudaStream_t s) {
-    tiles.clear();
+void GemmPlan::prepare(cudaStream_t s) const {
+    if (tab.dev.p) return;
+    std::vector<Tile> tiles;
     // heavy tasks first so that the tail of the grid is made of small tiles
     std::vector<int> order(tasks.size());
     std::vector<double> w(tasks.size());
@@ -260,9 +253,11 @@ void GemmPlan::finalize(cudaStream_t s) {
         for (int m0 = 0; m0 < t.m; m0 += tile_m)
             for (int n0 = 0; n0 < t.n; n0 += tile_n) tiles.push_back(Tile{ti, m0, n0});
     }
-    upload(dsegs, segs, s);
-    upload(dtasks, tasks, s);
-    upload(dtiles, tiles, s);
+    ntiles = tiles.size();
+    osegs = tab.add(segs);
+    otasks = tab.add(tasks);
+    otiles = tab.add(tiles);
+    tab.upload(s);
 }
 
 // (A_re + i a A_im)(B_re + i b B_im) = A_re B_re - a b A_im B_im + i (b A_re B_im + a A_im B_re)
@@ -316,9 +311,10 @@ void CombPlan::finalize(cudaStream_t s) {
         for (int r0 = 0; r0 < o.rows; r0 += COMB_TR)
             for (int c0 = 0; c0 < o.cols; c0 += COMB_TC) tiles.push_back(CombTile{int(i), r0, c0});
     }
-    upload(douts, outs, s);
-    upload(dterms, terms, s);
-    upload(dtiles, tiles, s);
+    oouts = tab.add(outs);
+    oterms = tab.add(terms);
+    otiles = tab.add(tiles);
+    tab.upload(s);
 }
 
 }  // namespace tn

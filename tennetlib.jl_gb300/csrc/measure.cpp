@@ -131,11 +131,9 @@ extern "C" int tn_mps_expect_local(tn_mps* mps, const double* op, double* out) {
         auto run = [&](GemmPlan& g, unsigned conj) {
             if (np == 2) {
                 GemmPlan c = complex_plan(g, conj);
-                c.finalize(st);
                 launch_gemm_f64(c, bs, st);
                 TN_CUDA(cudaStreamSynchronize(st));  // the plan goes out of scope
             } else {
-                g.finalize(st);
                 launch_gemm_f64(g, bs, st);
             }
         };
@@ -373,13 +371,9 @@ void overlap_impl(const tn_mps* a, const tn_mps* b, double* out, bool cx) {
             }
             if (cx) {  // <a|b>: a conjugated
                 GemmPlan c1 = complex_plan(g1, 0), c2 = complex_plan(g2, 1u << S_X);
-                c1.finalize(st);
-                c2.finalize(st);
                 launch_gemm_f64(c1, bs, st);
                 launch_gemm_f64(c2, bs, st);
             } else {
-                g1.finalize(st);
-                g2.finalize(st);
                 launch_gemm_f64(g1, bs, st);
                 launch_gemm_f64(g2, bs, st);
             }

@@ -114,8 +114,6 @@ void ov_left(tn_ctx* ctx, const tn_mps* a, const tn_mps* b, int i, const OvEnv& 
             g2.add_seg(S_X, j.xa->off, j.xa->ld, 1, S_T1, j.toff, Ein.da[j.ei], 0, Ein.da[j.ei]);
         }
     }
-    g1.finalize(st);
-    g2.finalize(st);
     Bases bs{};
     bs.p[S_L] = Ein.buf.d();
     bs.p[S_R] = Eout.buf.d();
@@ -164,8 +162,6 @@ void ov_right(tn_ctx* ctx, const tn_mps* a, const tn_mps* b, int i, const OvEnv&
             g2.add_seg(S_T1, j.toff, Eout.da[eo], 0, S_A, j.xb->off, j.xb->ld, 1, Ein.db[j.ei]);
         }
     }
-    g1.finalize(st);
-    g2.finalize(st);
     Bases bs{};
     bs.p[S_L] = Ein.buf.d();
     bs.p[S_R] = Eout.buf.d();
@@ -284,9 +280,6 @@ void proj_vectors2(tn_env* env, int p, const PhiLayout& ph) {
         if (g3.tasks.empty()) continue;
         env->projt1.alloc(size_t(std::max<int64_t>(t1, 1)) * 8, st);
         env->projt2.alloc(size_t(std::max<int64_t>(t2, 1)) * 8, st);
-        g1.finalize(st);
-        g2.finalize(st);
-        g3.finalize(st);
         Bases bs{};
         bs.p[S_L] = LM.buf.d();
         bs.p[S_R] = RM.buf.d();
@@ -345,8 +338,6 @@ void proj_vectors1(tn_env* env, int p, const SiteLayout& lay) {
         }
         if (g3.tasks.empty()) continue;
         env->projt1.alloc(size_t(std::max<int64_t>(t1, 1)) * 8, st);
-        g1.finalize(st);
-        g3.finalize(st);
         Bases bs{};
         bs.p[S_L] = LM.buf.d();
         bs.p[S_R] = RM.buf.d();

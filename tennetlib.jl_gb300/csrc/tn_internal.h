@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstring>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -56,6 +57,29 @@ struct DevBuf {
     void release();
     double* d() const { return static_cast<double*>(p); }
     template <class T> T* as() const { return static_cast<T*>(p); }
+};
+
+// The tables of a plan in one device buffer: collected on the host, one allocation and one copy
+// (the host's side is kept with the plan: the copy may still be reading it).
+struct Tables {
+    std::vector<unsigned char> host;
+    DevBuf dev;
+    template <class T>
+    size_t add(const std::vector<T>& v) {  // returns the table's offset
+        const size_t o = (host.size() + 15) & ~size_t(15);
+        host.resize(o + v.size() * sizeof(T));
+        if (!v.empty()) std::memcpy(host.data() + o, v.data(), v.size() * sizeof(T));
+        return o;
+    }
+    void upload(cudaStream_t s) {
+        dev.alloc(host.size(), s);
+        if (!host.empty())
+            TN_CUDA(cudaMemcpyAsync(dev.p, host.data(), host.size(), cudaMemcpyHostToDevice, s));
+    }
+    template <class T>
+    T* at(size_t o) const {
+        return reinterpret_cast<T*>(static_cast<unsigned char*>(dev.p) + o);
+    }
 };
 
 // ------------------------------------------------------------------------------------
@@ -168,21 +192,24 @@ struct CombTile {
 struct GemmPlan {
     std::vector<Seg> segs;
     std::vector<Task> tasks;
-    std::vector<Tile> tiles;
     double flops = 0;
-    int tile_m = 32, tile_n = 32;  // output tile of the FP64 kernel
-    DevBuf dsegs, dtasks, dtiles;
+    // the FP64 kernel's output tile, number of tiles and tables, made at its first launch (a
+    // plan that runs in split precision needs none of them)
+    mutable int tile_m = 32, tile_n = 32;
+    mutable size_t ntiles = 0, osegs = 0, otasks = 0, otiles = 0;
+    mutable Tables tab;
     void add_task(int cbuf, int64_t coff, int m, int n, int ldc, int accum = 0);
     void add_seg(int abuf, int64_t aoff, int lda, int ta, int bbuf, int64_t boff, int ldb,
                  int tb, int k, int sgn = 1);
-    void finalize(cudaStream_t s);  // builds tiles, uploads
+    void prepare(cudaStream_t s) const;  // tiles and tables, unless there already
 };
 struct CombPlan {
     std::vector<CombOut> outs;
     std::vector<CombTerm> terms;
     std::vector<CombTile> tiles;
     double flops = 0;
-    DevBuf douts, dterms, dtiles;
+    size_t oouts = 0, oterms = 0, otiles = 0;
+    Tables tab;
     void finalize(cudaStream_t s);
 };
 
@@ -224,8 +251,10 @@ struct SplitPlan {
     int64_t abytes = 0, bbytes = 0, ea_n = 0, eb_n = 0;
     int slices = 0;
     bool a_static = false, b_static = false, a_packed = false, b_packed = false;
-    DevBuf dtasks, ditems, dajobs, dbjobs, daks, dbks, apack, bpack, ea, eb;
-    // pack buffers used by the launches: the owned buffers above, or caller-provided
+    Tables tab;
+    size_t otasks = 0, oitems = 0, oajobs = 0, objobs = 0, oaks = 0, obks = 0;
+    DevBuf packs;
+    // pack buffers used by the launches: within the owned buffer above, or caller-provided
     // scratch (make_split with own_packs = false) of abytes / bbytes / 4 ea_n / 4 eb_n bytes
     uint8_t *ap = nullptr, *bp = nullptr;
     int *eap = nullptr, *ebp = nullptr;
@@ -237,6 +266,8 @@ int split_tile_bytes_b();
 int split_tile_rows_a();
 int split_tile_rows_b();
 int split_ktile();
+// whether operands with jobs of up to max_nkt k tiles are packed by the k-split kernels
+bool split_pack_needs_max(int max_nkt);
 // max_nkt: the largest k-tile count of a job; operands with long k are packed by the k-split
 // kernels, which need gmax (nrows 64-bit words of scratch, the exponent count of the operand)
 void launch_split_pack(const PackJob* jobs, int njobs, const KTileSrc* ksrc, const Bases& b,

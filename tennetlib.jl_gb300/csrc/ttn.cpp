@@ -217,7 +217,6 @@ struct TGroup {
 struct TPlan {
     GemmPlan g;
     std::unique_ptr<SplitPlan> sp;
-    bool finalized = false;
 };
 
 struct ProductPlan {    // H_eff x at one node
@@ -348,10 +347,6 @@ void tplan_run(TtnGroup& G, TPlan& p, int slices, int timecat) {
     if (p.g.tasks.empty()) return;
     tn_ctx* ctx = G.ctx;
     cudaStream_t st = ctx->stream;
-    if (!p.finalized) {
-        p.g.finalize(st);
-        p.finalized = true;
-    }
     const Bases bs = group_bases(G);
     const int e0 = ctx->timer.mark();
     if (slices == 0) {
@@ -916,7 +911,6 @@ ProjSrc proj_mapped(tn_ttn_env* e, TtnProj& P, int v, int skip, const Bases& bs,
         GemmPlan g;
         add_mode_tasks(g, dims, li, dout, dst.buf, dst.off,
                        {ModeIn{cur.buf, cur.off, S_A, P.eoff[eid]}}, 0);
-        g.finalize(st);
         launch_gemm_f64(g, bs, st);
         dims[li] = dout;
         cur = dst;
@@ -954,7 +948,6 @@ void proj_move(TtnGroup& G, tn_ttn_env* e, TtnProj& P, int v, int u) {
             g.add_seg(S_L, phi + q * Pr * Dp, int(Pr), 1, y.buf, y.off + q * Pr * Dm, int(Pr), 0,
                       int(Pr));
     }
-    g.finalize(st);
     launch_gemm_f64(g, bs, st);
     P.efrom[eid] = v;
 }
