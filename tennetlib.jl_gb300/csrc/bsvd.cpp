@@ -59,11 +59,11 @@ struct GemmRun {
         auto sp = make_split_plan(g, SVD_SLICES, st, true);
         launch_split_pack(sp->tab.at<PackJob>(sp->oajobs), (int)sp->ajobs.size(),
                           sp->tab.at<KTileSrc>(sp->oaks), bs, sp->ap, sp->eap, sp->slices,
-                          split_tile_rows_a(), st, sp->a_maxnkt,
+                          split_tile_rows_a(), sp->a_maxrows, st, sp->a_maxnkt,
                           sp->amax.as<unsigned long long>(), sp->ea_n);
         launch_split_pack(sp->tab.at<PackJob>(sp->objobs), (int)sp->bjobs.size(),
                           sp->tab.at<KTileSrc>(sp->obks), bs, sp->bp, sp->ebp, sp->slices,
-                          split_tile_rows_b(), st, sp->b_maxnkt,
+                          split_tile_rows_b(), sp->b_maxrows, st, sp->b_maxnkt,
                           sp->bmax.as<unsigned long long>(), sp->eb_n);
         launch_split_gemm(sp->tab.at<SplitItem>(sp->oitems), (int)sp->items.size(),
                           sp->tab.at<SplitTask>(sp->otasks), sp->ap, sp->bp, sp->eap, sp->ebp, bs,

@@ -305,8 +305,14 @@ std::unique_ptr<SplitPlan> make_split(const GemmPlan& g, int slices, bool a_stat
     sp->bbytes = boff;
     sp->ea_n = eao;
     sp->eb_n = ebo;
-    for (const auto& j : sp->ajobs) sp->a_maxnkt = std::max(sp->a_maxnkt, j.nkt);
-    for (const auto& j : sp->bjobs) sp->b_maxnkt = std::max(sp->b_maxnkt, j.nkt);
+    for (const auto& j : sp->ajobs) {
+        sp->a_maxnkt = std::max(sp->a_maxnkt, j.nkt);
+        sp->a_maxrows = std::max(sp->a_maxrows, int(j.rows));
+    }
+    for (const auto& j : sp->bjobs) {
+        sp->b_maxnkt = std::max(sp->b_maxnkt, j.nkt);
+        sp->b_maxrows = std::max(sp->b_maxrows, int(j.rows));
+    }
     if (split_pack_needs_max(sp->a_maxnkt)) sp->amax.alloc(size_t(std::max<int64_t>(eao, 1)) * 8, st);
     if (split_pack_needs_max(sp->b_maxnkt)) sp->bmax.alloc(size_t(std::max<int64_t>(ebo, 1)) * 8, st);
     sp->otasks = sp->tab.add(sp->tasks);
@@ -334,14 +340,16 @@ void run_split(tn_ctx* ctx, SplitPlan& sp, const Bases& bs, int* mma_ev0, int* m
     if (!sp.a_static || !sp.a_packed) {
         launch_split_pack(sp.tab.at<PackJob>(sp.oajobs), (int)sp.ajobs.size(),
                           sp.tab.at<KTileSrc>(sp.oaks), bs,
-                          sp.ap, sp.eap, sp.slices, split_tile_rows_a(), st, sp.a_maxnkt,
+                          sp.ap, sp.eap, sp.slices, split_tile_rows_a(),
+                          sp.a_maxrows, st, sp.a_maxnkt,
                           sp.amax.as<unsigned long long>(), sp.ea_n);
         sp.a_packed = true;
     }
     if (!sp.b_static || !sp.b_packed) {
         launch_split_pack(sp.tab.at<PackJob>(sp.objobs), (int)sp.bjobs.size(),
                           sp.tab.at<KTileSrc>(sp.obks), bs,
-                          sp.bp, sp.ebp, sp.slices, split_tile_rows_b(), st, sp.b_maxnkt,
+                          sp.bp, sp.ebp, sp.slices, split_tile_rows_b(),
+                          sp.b_maxrows, st, sp.b_maxnkt,
                           sp.bmax.as<unsigned long long>(), sp.eb_n);
         sp.b_packed = true;
     }

@@ -29,7 +29,9 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "tn_internal.h"
 
@@ -198,20 +200,33 @@ __device__ __forceinline__ double pow2(int e) {
     return __longlong_as_double(static_cast<long long>(1023 + e) << 52);
 }
 
-// double(x), exactly, on the integer pipe for zeros and normal numbers (a conversion holds the
-// FP64 pipe as long as an add does)
+// x, for arithmetic that has to stay in its branch: the compiler else takes it out and selects
+// between the results, and an FP64 operation holds the pipe for 64 clocks whether used or not
+__device__ __forceinline__ float branch_only(float x) {
+    asm volatile("" : "+f"(x));
+    return x;
+}
+__device__ __forceinline__ double branch_only(double x) {
+    asm volatile("" : "+d"(x));
+    return x;
+}
+
+// double(x) of a zero or normal number, exactly, on the integer pipe (a conversion holds the FP64
+// pipe as long as an add does)
+__device__ __forceinline__ bool plain(float x) {
+    const unsigned a = __float_as_uint(x) & 0x7fffffffu;
+    return a == 0u || a - 0x00800000u < 0x7f000000u;
+}
 __device__ __forceinline__ double widen(float x) {
     const unsigned u = __float_as_uint(x), a = u & 0x7fffffffu;
-    if (a - 0x00800000u >= 0x7f000000u && a != 0u) return double(x);  // subnormal, inf, NaN
     const unsigned hi = a ? (a >> 3) + 0x38000000u : 0u;
     return __hiloint2double(int(hi | (u & 0x80000000u)), int(u << 29));
 }
 
-// v * 2^e, exactly the product: on the exponent field while both v and the result are normal
+// v * 2^e, exactly the product, on the exponent field: v zero, or v and the result normal
 __device__ __forceinline__ double scale2(double v, int e) {
-    const int hi = __double2hiint(v), ex = (hi >> 20) & 0x7ff;
-    if (ex == 0 || ex == 0x7ff || unsigned(ex + e - 1) >= 2046u) return v * pow2(e);
-    return __hiloint2double(hi + (e << 20), __double2loint(v));
+    const int hi = __double2hiint(v), lo = __double2loint(v);
+    return __hiloint2double(((hi & 0x7fffffff) | lo) == 0 ? hi : hi + (e << 20), lo);
 }
 
 // ------------------------------------------------------------------------------------
@@ -220,7 +235,7 @@ __device__ __forceinline__ double scale2(double v, int e) {
 // k (split_ksteps; a charge block of 14 x 14 fills 16 rows and one step of four, a sixteenth of
 // its A tile).
 // ------------------------------------------------------------------------------------
-constexpr int PACK_THREADS = 256;
+constexpr int PACK_THREADS = 256, PACK_MAXTHREADS = 1024;
 constexpr int PACK_ROWS = 8;
 
 // 8-wide chunks of k tile t that are packed
@@ -228,18 +243,18 @@ __device__ __forceinline__ int pack_chunks(int t, int kvalid) {
     return t < SPLIT_KMASK ? 2 * ((kvalid + 15) / 16) : BKT / 8;
 }
 
-// Eight elements of row r (chunk ch of a k tile at tile0): balanced base-256 digits.
+// EL elements of row r (k = EL pr ... of a k tile at tile0): balanced base-256 digits.
 // x * 2^(8s - E) = sig * 2^(ex - 1075 + 8s - E), sig the 53-bit significand: the rounded
 // integer is sig shifted right by sh = 1075 + E - 8s - ex (round half away from zero), integer
 // pipe only.  mxb is the row's largest |x| as a bit pattern, 0 for an empty row.
-__device__ __forceinline__ void pack_digits(const long long (&v)[8], unsigned long long mxb,
-                                            int r, int ch, uint8_t* tile0, int tile_bytes,
-                                            int slices) {
+template <int SL, int EL>
+__device__ __forceinline__ void pack_digits(const long long (&v)[EL], unsigned long long mxb,
+                                            int r, int pr, uint8_t* tile0, int tile_bytes) {
     const int E = mxb ? int((mxb >> 52) & 0x7ff) - 1022 : 0;
-    const int base_sh = 1075 + E - 8 * slices;
-    __nv_bfloat16 dig[7][8];
+    const int base_sh = 1075 + E - 8 * SL;
+    __nv_bfloat16 dig[SL][EL];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < EL; ++q) {
         long long X = 0;
         const int ex = int((v[q] >> 52) & 0x7ff);
         if (mxb && ex) {  // subnormals are far below the row scale: they round to 0
@@ -250,10 +265,8 @@ __device__ __forceinline__ void pack_digits(const long long (&v)[8], unsigned lo
             else if (sh < 63) a = (m + (1LL << (sh - 1))) >> sh;
             X = v[q] < 0 ? -a : a;
         }
-        // compile-time slice indices keep dig[][] in registers
 #pragma unroll
-        for (int i = 6; i >= 1; --i) {
-            if (i >= slices) continue;
+        for (int i = SL - 1; i >= 1; --i) {
             int d = int(X & 255);
             if (d > 128) d -= 256;
             X = (X - d) >> 8;
@@ -261,26 +274,29 @@ __device__ __forceinline__ void pack_digits(const long long (&v)[8], unsigned lo
         }
         dig[0][q] = __float2bfloat16_rn(float(X));
     }
-    // swizzled position of (row r, chunk ch): 8-row atoms of 1024 bytes
-    const int off = (r >> 3) * 1024 + (r & 7) * 128 + ((ch ^ (r & 7)) << 4);
+    // swizzled position: 8-row atoms of 1024 bytes, 16-byte chunks XOR-ed with the row
+    const int ch = pr * EL / 8;
+    const int off = (r >> 3) * 1024 + (r & 7) * 128 + ((ch ^ (r & 7)) << 4) + pr * EL % 8 * 2;
+    using W = typename std::conditional<EL == 8, uint4, unsigned>::type;
+    static_assert(sizeof(W) == 2 * EL, "two or eight elements");
 #pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        if (i >= slices) continue;
-        uint4 w;
-        __builtin_memcpy(&w, dig[i], 16);
-        *reinterpret_cast<uint4*>(tile0 + int64_t(i) * tile_bytes + off) = w;
+    for (int i = 0; i < SL; ++i) {
+        W w;
+        __builtin_memcpy(&w, dig[i], sizeof(W));
+        *reinterpret_cast<W*>(tile0 + int64_t(i) * tile_bytes + off) = w;
     }
 }
 
-// the chunk's elements (zeros beyond the rows and valid k) and their largest |x|
-__device__ __forceinline__ unsigned long long pack_load(long long (&v)[8], const KTileSrc& ks,
+// EL elements from k = EL ch on (zeros beyond the rows and valid k) and their largest |x|
+template <int EL>
+__device__ __forceinline__ unsigned long long pack_load(long long (&v)[EL], const KTileSrc& ks,
                                                         const Bases& b, int row, bool live, int ch) {
     const long long* x = reinterpret_cast<const long long*>(b.p[ks.buf] + ks.off) +
                          int64_t(row) * ks.sr;
     unsigned long long mx = 0ull;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int k = ch * 8 + q;
+    for (int q = 0; q < EL; ++q) {
+        const int k = ch * EL + q;
         v[q] = live && k < ks.kvalid ? x[int64_t(k) * ks.sk] : 0ll;
         const unsigned long long a = (unsigned long long)v[q] & 0x7fffffffffffffffull;
         mx = a > mx ? a : mx;
@@ -289,46 +305,56 @@ __device__ __forceinline__ unsigned long long pack_load(long long (&v)[8], const
 }
 
 // A row tile is shared by CTAs of PACK_ROWS rows (gridDim.y), each packing all k tiles of its
-// rows: the row maxima stay within a CTA.  Work item: one row and one 8-wide chunk (16 bytes of
-// bf16) of one k tile; consecutive threads take consecutive rows so that the loads of a
-// column-major operand come in 64-byte pieces, and each thread keeps 8 loads in flight.  Bound
-// by load latency: 8 rows of up to four k tiles are one item per thread, whose elements stay in
-// registers between the maximum and the digits.  With 32 rows per CTA and whole tiles written
-// it took 12.4 us per launch on the blocks of a chi = 50 bond, now 6.2 us.
-__global__ void __launch_bounds__(PACK_THREADS)
+// rows: the row maxima stay within a CTA.  Work item: one row and two k, so that a k tile of 8
+// rows is one item for each of 256 threads; the block has the threads that the longest job has
+// items for (1024 at most), and the elements stay in registers between the maximum and the digits
+// while the k tiles do.  Consecutive threads take consecutive rows so that the loads of a
+// column-major operand come in 64-byte pieces.  Bound by latency, of the loads and of the
+// instructions: with eight elements a thread the straight code was four times as long and 64
+// threads of a CTA of 256 worked (one k tile; 31 us for the 4096 x 64 operands of four
+// instances; the blocks of a chi = 50 bond took 6.2 us, before that, with 32 rows per CTA and
+// whole tiles written, 12.4 us).
+template <int SL>
+__global__ void __launch_bounds__(PACK_MAXTHREADS)
 split_pack_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict__ ksrc,
                   const __grid_constant__ Bases b, uint8_t* __restrict__ out,
-                  int* __restrict__ expo, int slices, int tile_rows) {
+                  int* __restrict__ expo, int tile_rows) {
     __shared__ unsigned long long rowmax[PACK_ROWS];
     const PackJob jb = jobs[blockIdx.x];
     const int r0 = blockIdx.y * PACK_ROWS;
     if (r0 >= jb.rows) return;
     const int tile_bytes = tile_rows * BKT * 2;
-    constexpr int PER_TILE = PACK_ROWS * 8;         // (row, chunk) items per k tile
-    const int nitems = PER_TILE * jb.nkt;
+    constexpr int PER_TILE = PACK_ROWS * BKT / 2;  // (row, pair of k) items per k tile
+    const int nitems = PER_TILE * jb.nkt, nthr = blockDim.x;
     if (threadIdx.x < PACK_ROWS) rowmax[threadIdx.x] = 0ull;
     __syncthreads();
     const int rl = threadIdx.x % PACK_ROWS, r = r0 + rl;
     const bool live = r < jb.rows;
-    long long v[8];
-    // row maxima of |x| as IEEE bit patterns (integer compare, no FP64 pipe)
-    for (int it = threadIdx.x; it < nitems; it += PACK_THREADS) {
+    long long v[2];
+    // row maxima of |x| as IEEE bit patterns (integer compare, no FP64 pipe): over the four lanes
+    // of a row, then over the warps
+    for (int it = threadIdx.x; it < nitems; it += nthr) {
         const KTileSrc ks = ksrc[jb.kt0 + it / PER_TILE];
-        const unsigned long long mx =
+        unsigned long long mx =
             pack_load(v, ks, b, jb.row0 + r, live, (it % PER_TILE) / PACK_ROWS);
-        if (mx) atomicMax(&rowmax[rl], mx);
+#pragma unroll
+        for (int d = PACK_ROWS; d < 32; d *= 2) {
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, mx, d);
+            mx = o > mx ? o : mx;
+        }
+        if (mx && (threadIdx.x & 31) < PACK_ROWS) atomicMax(&rowmax[rl], mx);
     }
     __syncthreads();
     const unsigned long long mxb = rowmax[rl];
     if (threadIdx.x < PACK_ROWS && live)
         expo[jb.eoff + r] = mxb ? int((mxb >> 52) & 0x7ff) - 1022 : 0;
-    for (int it = threadIdx.x; it < nitems; it += PACK_THREADS) {
-        const int t = it / PER_TILE, ch = (it % PER_TILE) / PACK_ROWS;
+    for (int it = threadIdx.x; it < nitems; it += nthr) {
+        const int t = it / PER_TILE, pr = (it % PER_TILE) / PACK_ROWS;
         const KTileSrc ks = ksrc[jb.kt0 + t];
-        if (ch >= pack_chunks(t, ks.kvalid)) continue;
-        if (nitems > PACK_THREADS) pack_load(v, ks, b, jb.row0 + r, live, ch);
-        pack_digits(v, mxb, r, ch, out + jb.out_off + int64_t(t) * slices * tile_bytes, tile_bytes,
-                    slices);
+        if (pr >= 4 * pack_chunks(t, ks.kvalid)) continue;
+        if (nitems > nthr) pack_load(v, ks, b, jb.row0 + r, live, pr);
+        pack_digits<SL, 2>(v, mxb, r, pr, out + jb.out_off + int64_t(t) * SL * tile_bytes,
+                           tile_bytes);
     }
 }
 
@@ -363,11 +389,12 @@ split_rowmax_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict
         if (rowmax[r]) atomicMax(&gmax[jb.eoff + r], rowmax[r]);
 }
 
+template <int SL>
 __global__ void __launch_bounds__(PACK_THREADS)
 split_pack_part_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restrict__ ksrc,
                        const __grid_constant__ Bases b, uint8_t* __restrict__ out,
                        int* __restrict__ expo, const unsigned long long* __restrict__ gmax,
-                       int slices, int tile_rows, int kper) {
+                       int tile_rows, int kper) {
     const PackJob jb = jobs[blockIdx.x];
     const int t0 = blockIdx.y * kper;
     if (t0 >= jb.nkt) return;
@@ -376,12 +403,12 @@ split_pack_part_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restr
     const int rows8 = (jb.rows + 7) & ~7;
     const int per_tile = rows8 * 8;
     const int nitems = per_tile * (t1 - t0);
-    if (blockIdx.y == 0)
+    if (blockIdx.y == 0 && blockIdx.z == 0)
         for (int r = threadIdx.x; r < jb.rows; r += blockDim.x) {
             const unsigned long long m = gmax[jb.eoff + r];
             expo[jb.eoff + r] = m ? int((m >> 52) & 0x7ff) - 1022 : 0;
         }
-    for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
+    for (int it = blockIdx.z * blockDim.x + threadIdx.x; it < nitems; it += gridDim.z * blockDim.x) {
         const int t = t0 + it / per_tile, rem = it % per_tile;
         const int r = rem % rows8, ch = rem / rows8;
         const KTileSrc ks = ksrc[jb.kt0 + t];
@@ -390,8 +417,8 @@ split_pack_part_kernel(const PackJob* __restrict__ jobs, const KTileSrc* __restr
         const unsigned long long mxb = live ? gmax[jb.eoff + r] : 0ull;
         long long v[8];
         pack_load(v, ks, b, jb.row0 + r, live, ch);
-        pack_digits(v, mxb, r, ch, out + jb.out_off + int64_t(t) * slices * tile_bytes, tile_bytes,
-                    slices);
+        pack_digits<SL, 8>(v, mxb, r, ch, out + jb.out_off + int64_t(t) * SL * tile_bytes,
+                           tile_bytes);
     }
 }
 
@@ -592,17 +619,28 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
                 if (!mbar_wait(&sh->tfull[buf], (chunk >> 1) & 1, err, serr)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;");
                 const uint32_t tbase = tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * NACC * BN + h * 16);
-#pragma unroll
+                // (the two column groups in a loop, its registers swapped after each pass: straight
+                // code of this length waits for its instructions)
+#pragma unroll 1
                 for (int g = 0; g < 2; ++g) {
-                    if (16 * h + 32 * g >= ncol) continue;
-                    float v[NACC][16];
+                    if (16 * h + 32 * g < ncol) {
+                        float v[NACC][16];
 #pragma unroll
-                    for (int l = 0; l < NACC; ++l) tmem_ld16(tbase + l * BN + 32 * g, v[l]);
-                    tmem_wait(v);
+                        for (int l = 0; l < NACC; ++l) tmem_ld16(tbase + l * BN + 32 * g, v[l]);
+                        tmem_wait(v);
 #pragma unroll
-                    for (int l = 0; l < NACC; ++l)
+                        for (int l = 0; l < NACC; ++l)
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) df_add(hi[16 * g + c], lo[16 * g + c], v[l][c]);
+                            for (int c = 0; c < 16; ++c) df_add(hi[c], lo[c], v[l][c]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) {
+                        const float th = hi[c], tl = lo[c];
+                        hi[c] = hi[c + 16];
+                        lo[c] = lo[c + 16];
+                        hi[c + 16] = th;
+                        lo[c + 16] = tl;
+                    }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;");
                 __syncwarp();
@@ -611,21 +649,55 @@ split_gemm_kernel(const SplitItem* __restrict__ items, int nitems,
             if (!ok) break;
             if (ncol == 0) continue;
             double* C = b.p[tk.cbuf] + tk.coff + gr + int64_t(item.nt * BN) * tk.ldc;
-            // (left at the block's last column: the code of the 32 columns is long, and stepping
-            // over unused ones costs an instruction fetch each)
+            // Four columns at a time, their chains (exponent, widening, sum, scaling) side by side,
+            // in a loop that takes columns 0 to 3 of the registers and moves the rest down.  One
+            // FP64 operation a column, two with accumulation; what the integer forms do not cover
+            // (subnormals, infinities, NaN, exponents beyond any product of normal operands) takes
+            // a branch of its own.  One column after the other, each with a branch at every special
+            // value, took 470 clocks a column; this takes 350 (230 eight at a time, which lose more
+            // on the blocks of a few columns than they gain on the wide ones: 281 against 279 ms
+            // on a chi = 50 chain).
+            // The lanes beyond the block hold whatever the accumulators did: zero here.
+            constexpr int GC = 4;
+            if (gr >= tk.m) {
 #pragma unroll
-            for (int g = 0; g < 2; ++g)
+                for (int c = 0; c < HC; ++c) { hi[c] = 0.f; lo[c] = 0.f; }
+            }
+#pragma unroll 1
+            for (int c0 = 0; c0 < HC; c0 += GC) {
+                const int tc = c0 + 16 * h + (c0 & 16);  // first column of the four
+                if (tc >= ncol) break;
+                const int nc = gr < tk.m ? ncol - tc : 0;  // columns that this lane stores
+                double* out = C + int64_t(tc) * tk.ldc;
+                double old[GC], v[GC];
+                if (tk.accum)
 #pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const int c = 16 * g + k, tc = k + 16 * h + 32 * g;
-                    if (tc >= ncol) break;
-                    const int e = er + __shfl_sync(0xffffffffu, ec, c) - 16;
-                    const double v = scale2(widen(hi[c]) + widen(lo[c]), e);
-                    if (gr < tk.m) {
-                        double* out = C + int64_t(tc) * tk.ldc;
-                        *out = tk.accum ? *out + v : v;
-                    }
+                    for (int j = 0; j < GC; ++j) old[j] = j < nc ? out[int64_t(j) * tk.ldc] : 0.0;
+                int e[GC];
+                bool fast = true;
+#pragma unroll
+                for (int j = 0; j < GC; ++j) {
+                    e[j] = er + __shfl_sync(0xffffffffu, ec, c0 + j) - 16;
+                    fast = fast && (j >= ncol - tc || (plain(hi[j]) && plain(lo[j]) &&
+                                                       unsigned(e[j] + 800) <= 1600u));
                 }
+                if (__all_sync(0xffffffffu, fast)) {
+#pragma unroll
+                    for (int j = 0; j < GC; ++j) v[j] = scale2(widen(hi[j]) + widen(lo[j]), e[j]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < GC; ++j)
+                        v[j] = (double(branch_only(hi[j])) + double(branch_only(lo[j]))) * pow2(e[j]);
+                }
+                if (tk.accum)
+#pragma unroll
+                    for (int j = 0; j < GC; ++j) v[j] = branch_only(old[j]) + v[j];
+#pragma unroll
+                for (int j = 0; j < GC; ++j)
+                    if (j < nc) out[int64_t(j) * tk.ldc] = v[j];
+#pragma unroll
+                for (int c = 0; c + GC < HC; ++c) { hi[c] = hi[c + GC]; lo[c] = lo[c + GC]; }
+            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -647,14 +719,19 @@ constexpr int KPER = 2;  // k tiles per CTA of the k-split pack
 bool split_pack_needs_max(int max_nkt) { return max_nkt > 2 * KPER; }
 
 void launch_split_pack(const PackJob* jobs, int njobs, const KTileSrc* ksrc, const Bases& b,
-                       uint8_t* out, int* expo, int slices, int tile_rows, cudaStream_t s,
-                       int max_nkt, unsigned long long* gmax, int64_t nrows) {
+                       uint8_t* out, int* expo, int slices, int tile_rows, int max_rows,
+                       cudaStream_t s, int max_nkt, unsigned long long* gmax, int64_t nrows) {
     if (njobs <= 0) return;
     TN_REQUIRE(slices >= 4 && slices <= 7, "split precision needs 4..7 slices");
     TN_REQUIRE(tile_rows <= BM, "pack tile taller than the A tile");
     if (!split_pack_needs_max(max_nkt) || !gmax) {
-        const dim3 g(njobs, (tile_rows + PACK_ROWS - 1) / PACK_ROWS);
-        split_pack_kernel<<<g, PACK_THREADS, 0, s>>>(jobs, ksrc, b, out, expo, slices, tile_rows);
+        const dim3 g(njobs, (max_rows + PACK_ROWS - 1) / PACK_ROWS);
+        const int nthr = std::min(PACK_MAXTHREADS, PACK_ROWS * BKT / 2 * std::max(max_nkt, 1));
+        auto* kernel = slices == 4   ? split_pack_kernel<4>
+                       : slices == 5 ? split_pack_kernel<5>
+                       : slices == 6 ? split_pack_kernel<6>
+                                     : split_pack_kernel<7>;
+        kernel<<<g, nthr, 0, s>>>(jobs, ksrc, b, out, expo, tile_rows);
         TN_CUDA(cudaGetLastError());
         count_launch();
         return;
@@ -663,8 +740,14 @@ void launch_split_pack(const PackJob* jobs, int njobs, const KTileSrc* ksrc, con
     TN_CUDA(cudaMemsetAsync(gmax, 0, size_t(nrows) * sizeof(unsigned long long), s));
     split_rowmax_kernel<<<g, PACK_THREADS, 0, s>>>(jobs, ksrc, b, gmax, KPER);
     TN_CUDA(cudaGetLastError());
-    split_pack_part_kernel<<<g, PACK_THREADS, 0, s>>>(jobs, ksrc, b, out, expo, gmax, slices,
-                                                      tile_rows, KPER);
+    // two items a thread
+    const int nz = std::max(1, (max_rows + 7) / 8 * 8 * (BKT / 8) * KPER / (2 * PACK_THREADS));
+    auto* kernel = slices == 4   ? split_pack_part_kernel<4>
+                   : slices == 5 ? split_pack_part_kernel<5>
+                   : slices == 6 ? split_pack_part_kernel<6>
+                                 : split_pack_part_kernel<7>;
+    kernel<<<dim3(g.x, g.y, nz), PACK_THREADS, 0, s>>>(jobs, ksrc, b, out, expo, gmax, tile_rows,
+                                                       KPER);
     TN_CUDA(cudaGetLastError());
     count_launch(2);
 }

@@ -259,6 +259,7 @@ struct SplitPlan {
     uint8_t *ap = nullptr, *bp = nullptr;
     int *eap = nullptr, *ebp = nullptr;
     int a_maxnkt = 0, b_maxnkt = 0;   // longest k (in tiles) of a pack job
+    int a_maxrows = 0, b_maxrows = 0;  // most rows of one
     DevBuf amax, bmax;                // row maxima scratch of the k-split pack
 };
 int split_tile_bytes_a();
@@ -268,11 +269,11 @@ int split_tile_rows_b();
 int split_ktile();
 // whether operands with jobs of up to max_nkt k tiles are packed by the k-split kernels
 bool split_pack_needs_max(int max_nkt);
-// max_nkt: the largest k-tile count of a job; operands with long k are packed by the k-split
+// max_rows, max_nkt: the largest row and k-tile count of a job; operands with long k are packed by the k-split
 // kernels, which need gmax (nrows 64-bit words of scratch, the exponent count of the operand)
 void launch_split_pack(const PackJob* jobs, int njobs, const KTileSrc* ksrc, const Bases& b,
-                       uint8_t* out, int* expo, int slices, int tile_rows, cudaStream_t s,
-                       int max_nkt = 0, unsigned long long* gmax = nullptr, int64_t nrows = 0);
+                       uint8_t* out, int* expo, int slices, int tile_rows, int max_rows,
+                       cudaStream_t s, int max_nkt, unsigned long long* gmax, int64_t nrows);
 void launch_split_gemm(const SplitItem* items, int nitems, const SplitTask* tasks,
                        const uint8_t* apack, const uint8_t* bpack, const int* ea, const int* eb,
                        const Bases& b, int slices, int* err, int nsm, cudaStream_t s);
