@@ -1200,7 +1200,9 @@ void run_qr_move(TtnGroup& G, int v, int u, int maxdim, int mindim = 1, double c
     if (!small.empty()) {
         upload_descs(G, G.d_qr, small);
         const int q0 = G.ctx->timer.mark();
-        launch_qr_small(G.d_qr.as<QrDesc>(), int(small.size()), st);
+        size_t shm = 0;
+        for (const QrDesc& q : small) shm = std::max(shm, qr_cluster_smem(q.m, q.n));
+        launch_qr_small(G.d_qr.as<QrDesc>(), int(small.size()), shm, st);
         G.ctx->timer.add(T_QRPANEL, q0, G.ctx->timer.mark());
     }
     // a truncating move changes the dimensions: its plan is built for this move only
