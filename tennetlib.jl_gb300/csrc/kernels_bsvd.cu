@@ -1128,8 +1128,8 @@ int bsvd_panel_width(int mmax) {
 }
 
 // Column blocks as wide as the registers of the resident column and the shared memory of the
-// staged columns allow: n B <= 512 RM and 2 B n sizeof(T) <= SMEM_MAX (FP32: B in {16, 8, 4},
-// double-float: B in {16, 8, 4, 2}, the polish with half the FP32 width or more).
+// staged columns allow: n B <= 512 RM and 2 B n sizeof(T) <= SMEM_MAX (double-float: B in
+// {16, 8, 4, 2}; FP32, only beyond bj32_kernel's columns: B in {8, 4}).
 int bsvd_max_n() { return 3568; }
 
 // The FP32 presolve takes bj32_kernel while its staged columns fit shared memory
@@ -1197,7 +1197,6 @@ int bsvd_jacobi_capacity(int maxn, int precision) {
         return nsm * per;
     }
     switch (bsvd_jacobi_block(maxn, precision) + 100 * precision) {
-        case 16: return bj_capacity<float, 16>(maxn);
         case 8: return bj_capacity<float, 8>(maxn);
         case 4: return bj_capacity<float, 4>(maxn);
         case 116: return bj_capacity<df2, 16>(maxn);
@@ -1227,7 +1226,6 @@ void launch_bsvd_jacobi(const BjDesc* d, int nd, int nctas, int maxn, int precis
         return;
     }
     switch (bsvd_jacobi_block(maxn, precision) + 100 * precision) {
-        case 16: bj_launch<float, 16>(d, nd, nctas, maxn, 2.0e-5f, 30, 0, err, s); break;
         case 8: bj_launch<float, 8>(d, nd, nctas, maxn, 2.0e-5f, 30, 0, err, s); break;
         case 4: bj_launch<float, 4>(d, nd, nctas, maxn, 2.0e-5f, 30, 0, err, s); break;
         case 116: bj_launch<df2, 16>(d, nd, nctas, maxn, tdf, 30, 1, err, s); break;
