@@ -409,6 +409,13 @@ void add_mode_tasks(GemmPlan& g, const std::vector<int>& dims, int leg, int dout
     }
 }
 
+// Chunks of a long k.  The outputs of these products are a few tiles (64 x 64 for 4096 rows) and a
+// tile's k tiles run one after the other, so few chunks leave most SMs idle: pieces of 256 (four k
+// tiles, which the pack still takes in one launch) up to 32 of them, where the sums over the
+// partials would take over.  In pieces of 512 (rows of a QR panel) and 2048 (link contractions)
+// the products of four 4096 x 64 matrices took 46 us on 32 CTAs and 93 us on 24.
+int64_t k_chunks(int64_t k) { return std::max<int64_t>(1, std::max(k / 2048, std::min<int64_t>(32, k / 256))); }
+
 // T (D x D, at tbuf/toff) = contraction of phi and Y over every leg but `leg`;
 // k is split in chunks written to partial buffers and summed by `comb` when large
 void add_env_contraction(GemmPlan& g, CombPlan& comb, const std::vector<int>& dims, int leg,
@@ -421,7 +428,7 @@ void add_env_contraction(GemmPlan& g, CombPlan& comb, const std::vector<int>& di
     const int64_t per_unit = Q == 1 || P == 1 ? 1 : P;
     const int64_t ktot = units * per_unit;
     int nch = 1;
-    if (ktot >= 4096 && D >= 16) nch = int(std::min<int64_t>(nchunk_max, ktot / 2048));
+    if (ktot >= 1024 && D >= 16) nch = int(std::min<int64_t>(nchunk_max, k_chunks(ktot)));
     nch = std::max(1, std::min<int>(nch, int(units)));
     const int64_t per = (units + nch - 1) / nch;
     std::vector<int64_t> parts;
@@ -1037,7 +1044,7 @@ std::unique_ptr<QrPlan> build_qr_plan(TtnGroup& G, int v, int u, const std::vect
                     // Wt = A_trail^T V (split over rows; nt x pb so that the long side is M),
                     // W2 = (-T)^T Wt^T, A_trail += V W2
                     const int64_t atr = aoff + p0 + int64_t(p0 + pb) * m;
-                    const int nch = int(std::min<int64_t>(e->nchunk_q, std::max<int64_t>(1, rows / 512)));
+                    const int nch = int(std::min<int64_t>(e->nchunk_q, std::max(k_chunks(rows), rows / 512)));
                     const int64_t per = (rows + nch - 1) / nch;
                     std::vector<int64_t> parts;
                     for (int c = 0; c < nch; ++c) {
@@ -1073,7 +1080,7 @@ std::unique_ptr<QrPlan> build_qr_plan(TtnGroup& G, int v, int u, const std::vect
             const int64_t vo = e->wbase + e->w_qv;
             const int64_t cap = std::max<int64_t>(1, int64_t(e->nchunk_q) * HH_B * e->dmax /
                                                          (int64_t(kmin) * kmin));
-            const int nch = int(std::min<int64_t>(cap, std::max<int64_t>(1, m / 512)));
+            const int nch = int(std::min<int64_t>(cap, std::max(k_chunks(m), m / 512)));
             const int64_t per = (m + nch - 1) / nch;
             std::vector<int64_t> parts;
             for (int c = 0; c < nch; ++c) {
