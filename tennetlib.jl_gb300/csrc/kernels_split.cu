@@ -762,10 +762,12 @@ void launch_split_gemm(const SplitItem* items, int nitems, const SplitTask* task
                    : slices == 5 ? split_gemm_kernel<5>
                    : slices == 6 ? split_gemm_kernel<6>
                                  : split_gemm_kernel<7>;
-    static std::atomic<bool> attr[8];
-    if (!attr[slices]) {
+    static std::atomic<bool> attr[8][64];  // per device: the attribute belongs to its context
+    int dev = 0;
+    TN_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !attr[slices][dev]) {
         TN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
-        attr[slices] = true;
+        if (dev >= 0 && dev < 64) attr[slices][dev] = true;
     }
     const int grid = nitems < nsm ? nitems : nsm;
     kernel<<<grid, THREADS, shm, s>>>(items, nitems, tasks, apack, bpack, ea, eb, b, err);

@@ -11,7 +11,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 
 #include "reduce.cuh"
 #include "ttn_internal.h"
@@ -585,12 +584,14 @@ __device__ __forceinline__ bool inst_barrier(unsigned* bar, unsigned target, int
 //
 // Bound by the FP64 pipe and the chain of a column (sums, barrier, totals, root and divisions,
 // update), not by memory.  A warp-wide FP64 operation takes 64 clocks, so a thread works on 8
-// columns of one row (4 column groups x 2 groups of 32 rows per CTA, 64 rows in flight), warp sums
+// columns of one row (4 even column groups, one per sub-partition, x 2 groups of 32 rows per CTA),
+// warp sums
 // are merged (9 adds for 8 columns instead of 40), and the two divisions of the reflector go to
 // two warps.  With one row of 32 columns per thread and plain butterflies (160 adds) a panel of
 // four 4096 x 64 matrices took 658 us, now 315 (four 64-site trees at chi = 64: 751 -> 675 ms a sweep).
 constexpr int HP_COLS = 8, HP_CG = HH_B / HP_COLS, HP_RG = BT / 32 / HP_CG;
 constexpr int HP_ROWS = 32 * HP_RG;  // rows of a CTA in one pass
+constexpr int HP_TALL = 1024;
 __global__ void __launch_bounds__(BT, 2)
 hh_panel_coop_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* err) {
     constexpr int W1 = HH_B + 1;
@@ -619,13 +620,16 @@ hh_panel_coop_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* e
     double* parts = D.part;                          // 2 x G x W1: [sigma^2, s_0, s_1, ...]
     double* pubs = D.part + 2 * int64_t(G) * W1;     // 2 x W1: A[j, j], A[j, j+1], ...
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int cg = wid % HP_CG, rg = wid / HP_CG, c0 = cg * HP_COLS;
+    const int cg = wid % HP_CG, rg = wid / HP_CG;
     unsigned nb = 0;
     for (int j = p0; j < pe; ++j) {
         const int buf = j & 1;
         double* col = D.A + int64_t(j) * m;
         const int nk = pe - j - 1;
-        const bool mine = c0 < nk;  // this warp's column group has columns
+        // the columns right of j in HP_CG even groups, one per sub-partition
+        const int cpg = (nk + HP_CG - 1) / HP_CG, c0 = cg * cpg;
+        const int nc = cpg < nk - c0 ? cpg : nk - c0;  // columns of this warp's group
+        const bool mine = nc > 0;
         double ss = 0.0;
         double acc[HP_COLS];
 #pragma unroll
@@ -638,7 +642,7 @@ hh_panel_coop_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* e
                 const double* arow = D.A + i + int64_t(j + 1 + c0) * m;
 #pragma unroll
                 for (int c = 0; c < HP_COLS; ++c)
-                    if (c0 + c < nk) acc[c] = fma(x, arow[int64_t(c) * m], acc[c]);
+                    if (c < nc) acc[c] = fma(x, arow[int64_t(c) * m], acc[c]);
             }
         if (cg == 0) {
             ss = warp_sum(ss);
@@ -646,7 +650,8 @@ hh_panel_coop_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* e
         }
         if (mine) {
             const double v = warp_sum_multi<HP_COLS>(acc, lane);
-            if (warp_sum_owner<HP_COLS>(lane)) red[rg][1 + c0 + warp_sum_index<HP_COLS>(lane)] = v;
+            const int c = warp_sum_index<HP_COLS>(lane);
+            if (warp_sum_owner<HP_COLS>(lane) && c < nc) red[rg][1 + c0 + c] = v;
         }
         __syncthreads();
         if (threadIdx.x <= nk) {
@@ -696,12 +701,129 @@ hh_panel_coop_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* e
                 double* arow = D.A + i + int64_t(j + 1 + c0) * m;
 #pragma unroll
                 for (int c = 0; c < HP_COLS; ++c)
-                    if (c0 + c < nk) arow[int64_t(c) * m] = fma(-v, wsh[c0 + c], arow[int64_t(c) * m]);
+                    if (c < nc) arow[int64_t(c) * m] = fma(-v, wsh[c0 + c], arow[int64_t(c) * m]);
             }
         __syncthreads();  // every column group has read column j
         if (cg == 0)
             for (int64_t i = r0 + 32 * rg + lane; i < r1; i += HP_ROWS)
                 if (i >= j) col[i] = i == j ? beta : col[i] * scale;
+        if (g == 0 && threadIdx.x == 0) D.tau[j] = tau;
+        __syncthreads();
+    }
+}
+
+// The same with one row of all 32 columns per thread: more loads in flight per warp, column j read
+// once, and the adds of the sums spread over many rows, for CTAs of more than HP_TALL rows.  There
+// the panel is bound by memory and the FP64 pipe, not by the chain of a column: 32 trees with
+// matrices up to 65536 x 256 (about 3000 rows a CTA) took 5.6 s of panels a sweep with it, 7.7 s
+// with the other; at 54 rows a CTA (four 4096 x 64 matrices) the other takes 305 us, this 658.
+__global__ void __launch_bounds__(BT, 2)
+hh_panel_tall_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* err) {
+    constexpr int W1 = HH_B + 1;
+    __shared__ double red[BT / 32][W1];
+    __shared__ double tot[W1];
+    __shared__ double wsh[HH_B];
+    __shared__ double sc[3];
+    __shared__ int s_fail;
+    int inst = -1;
+    for (int i = 0; i < ninst; ++i)
+        if (int(blockIdx.x) >= descs[i].cta0 && int(blockIdx.x) < descs[i].cta0 + descs[i].ncta) inst = i;
+    if (inst < 0) return;
+    const HhDesc& D = descs[inst];
+    if (p0 >= D.kmin) return;  // uniform over the instance's CTAs
+    const int G = D.ncta, g = int(blockIdx.x) - D.cta0;
+    // test hook (tn_ctx_inject_wait_timeout, code 3): the first CTA of the first instance leaves
+    // before its first barrier, so that the other CTAs' barrier waits run out
+    if (threadIdx.x == 0) s_fail = (inst == 0 && g == 0 && atomicCAS(err + 1, 3, 0) == 3) ? 1 : 0;
+    __syncthreads();
+    if (s_fail) return;
+    const int pe = (p0 + HH_B) < D.kmin ? (p0 + HH_B) : D.kmin;
+    const int64_t m = D.m;
+    const int64_t chunk = (m - p0 + G - 1) / G;
+    const int64_t r0 = p0 + int64_t(g) * chunk;
+    const int64_t r1 = (r0 + chunk) < m ? (r0 + chunk) : m;
+    double* parts = D.part;                          // 2 x G x W1: [sigma^2, s_0, s_1, ...]
+    double* pubs = D.part + 2 * int64_t(G) * W1;     // 2 x W1: A[j, j], A[j, j+1], ...
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned nb = 0;
+    for (int j = p0; j < pe; ++j) {
+        const int buf = j & 1;
+        double* col = D.A + int64_t(j) * m;
+        const int nk = pe - j - 1;
+        double ss = 0.0;
+        double acc[HH_B];
+#pragma unroll
+        for (int c = 0; c < HH_B; ++c) acc[c] = 0.0;
+        for (int64_t i = (r0 > j + 1 ? r0 : j + 1) + threadIdx.x; i < r1; i += BT) {
+            const double x = col[i];
+            ss = fma(x, x, ss);
+            const double* arow = D.A + i + int64_t(j + 1) * m;
+            // groups of 8 columns past nk are skipped whole
+#pragma unroll
+            for (int cg = 0; cg < HH_B; cg += 8) {
+                if (cg >= nk) break;
+#pragma unroll
+                for (int c = cg; c < cg + 8; ++c)
+                    if (c < nk) acc[c] = fma(x, arow[int64_t(c) * m], acc[c]);
+            }
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) red[wid][0] = ss;
+#pragma unroll
+        for (int c = 0; c < HH_B; ++c) {
+            if (c >= ((nk + 7) & ~7)) break;
+            const double v = warp_sum(acc[c]);
+            if (lane == 0) red[wid][1 + c] = v;
+        }
+        __syncthreads();
+        if (threadIdx.x <= nk) {
+            double t = 0.0;
+            for (int w = 0; w < BT / 32; ++w) t += red[w][threadIdx.x];
+            parts[(int64_t(buf) * G + g) * W1 + threadIdx.x] = t;
+            if (j >= r0 && j < r1) pubs[buf * W1 + threadIdx.x] = col[j + int64_t(threadIdx.x) * m];
+        }
+        if (!inst_barrier(D.bar, (++nb) * unsigned(G), err, &s_fail)) return;
+        // totals: every CTA sums the G partials in the same fixed order (lane-strided, then a
+        // warp tree), so the reflectors are identical everywhere
+        // (L2 loads: the partials were written by other SMs before the barrier's fences)
+        const double* pall = parts + int64_t(buf) * G * W1;
+        const double* pub = pubs + buf * W1;
+        for (int c = wid; c <= nk; c += BT / 32) {
+            double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
+            int b = lane;
+            for (; b + 96 < G; b += 128) {
+                t0 += __ldcg(pall + int64_t(b) * W1 + c);
+                t1 += __ldcg(pall + int64_t(b + 32) * W1 + c);
+                t2 += __ldcg(pall + int64_t(b + 64) * W1 + c);
+                t3 += __ldcg(pall + int64_t(b + 96) * W1 + c);
+            }
+            for (; b < G; b += 32) t0 += __ldcg(pall + int64_t(b) * W1 + c);
+            const double t = warp_sum((t0 + t1) + (t2 + t3));
+            if (lane == 0) tot[c] = t;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double tau, scale, beta;
+            make_reflector(__ldcg(pub), tot[0], tau, scale, beta);
+            sc[0] = tau;
+            sc[1] = scale;
+            sc[2] = beta;
+        }
+        __syncthreads();
+        const double tau = sc[0], scale = sc[1], beta = sc[2];
+        if (threadIdx.x < nk) wsh[threadIdx.x] = tau * (__ldcg(pub + 1 + threadIdx.x) + scale * tot[1 + threadIdx.x]);
+        __syncthreads();
+        const int64_t i0 = r0 > j ? r0 : j;
+        if (nk > 0) {
+            for (int64_t i = i0 + threadIdx.x; i < r1; i += BT) {
+                const double v = i == j ? 1.0 : col[i] * scale;
+                for (int c = 0; c < nk; ++c) {
+                    double* a = D.A + i + int64_t(j + 1 + c) * m;
+                    *a = fma(-v, wsh[c], *a);
+                }
+            }
+        }
+        for (int64_t i = i0 + threadIdx.x; i < r1; i += BT) col[i] = i == j ? beta : col[i] * scale;
         if (g == 0 && threadIdx.x == 0) D.tau[j] = tau;
         __syncthreads();
     }
@@ -960,12 +1082,8 @@ size_t qr_cluster_smem(int64_t m, int64_t n) {
 void launch_qr_small(const QrDesc* d, int ninst, size_t shm, cudaStream_t s) {
     if (ninst <= 0) return;
     if (shm <= size_t(200) * 1024) {
-        static std::atomic<bool> attr;
-        if (!attr) {
-            TN_CUDA(cudaFuncSetAttribute(qr_cluster_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            attr = true;
-        }
+        TN_CUDA(cudaFuncSetAttribute(qr_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(shm)));
         qr_cluster_kernel<<<ninst * QC_CL, BT, shm, s>>>(d);
     } else {
         qr_small_kernel<<<ninst, 1024, 0, s>>>(d);
@@ -992,26 +1110,32 @@ void launch_hh_column(const HhDesc* d, int ninst, int64_t mmax, int j, int p0, i
 // co-resident CTAs of the cooperative panel kernel on the current device (cached per device)
 int hh_coop_rows() { return HP_ROWS; }
 
-int hh_coop_capacity() {
+int hh_tall_rows() { return HP_TALL; }
+
+int hh_coop_capacity(bool tall) {
     constexpr int MAXDEV = 64;
-    static int cap[MAXDEV] = {};
+    static int caps[2][MAXDEV] = {};
+    int* cap = caps[tall ? 1 : 0];
     int dev = 0;
     TN_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= MAXDEV) throw Error(-1, "device index out of range");
     if (cap[dev] <= 0) {
         int nsm = 0, per = 0;
         TN_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        TN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, hh_panel_coop_kernel, BT, 0));
+        if (tall)
+            TN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, hh_panel_tall_kernel, BT, 0));
+        else
+            TN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, hh_panel_coop_kernel, BT, 0));
         cap[dev] = nsm * per;
     }
     return cap[dev];
 }
 
-void launch_hh_panel_coop(const HhDesc* d, int ninst, int nctas, int p0, int* err,
+void launch_hh_panel_coop(const HhDesc* d, int ninst, int nctas, bool tall, int p0, int* err,
                           cudaStream_t s) {
     void* args[] = {(void*)&d, (void*)&ninst, (void*)&p0, (void*)&err};
-    TN_CUDA(cudaLaunchCooperativeKernel((const void*)hh_panel_coop_kernel, dim3(nctas), dim3(BT),
-                                        args, 0, s));
+    const void* kernel = tall ? (const void*)hh_panel_tall_kernel : (const void*)hh_panel_coop_kernel;
+    TN_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(nctas), dim3(BT), args, 0, s));
     count_launch();
 }
 
@@ -1019,7 +1143,9 @@ void launch_hh_panel_end(const HhDesc* d, int ninst, int64_t mmax, int p0, int p
                          cudaStream_t s) {
     hh_build_v_kernel<<<dim3(grid_x(mmax * pb, 2 * TTN_PARTS), ninst), BT, 0, s>>>(d, p0, pb);
     TN_CUDA(cudaGetLastError());
-    const int parts = std::max(8, TTN_PARTS / ninst);  // one per SM (TTN_PARTS) over all instances
+    // one per SM (TTN_PARTS) over all instances, more where that leaves a block over 512 rows
+    const int parts = int(std::max<int64_t>(std::max(8, TTN_PARTS / ninst),
+                                            std::min<int64_t>(TTN_PARTS, mmax / 512)));
     const int g = int(std::min<int64_t>(std::max<int64_t>((mmax + 63) / 64, 1), parts));
     hh_gram_t_kernel<<<dim3(g, ninst), HH_B * HH_B, 0, s>>>(d, p0, pb);
     TN_CUDA(cudaGetLastError());

@@ -1219,20 +1219,26 @@ void run_qr_move(TtnGroup& G, int v, int u, int maxdim, int mindim = 1, double c
     QrPlan& QP = any_trunc ? *once : qr_plan(G, v, u, blocked, kmins);
     if (!hh.empty()) {
         // CTAs of the cooperative panel kernel, in proportion to the rows of each matrix
-        const int cap = hh_coop_capacity();
         const int nh0 = int(hh.size());
-        bool coop = nh0 <= cap;
-        if (coop) {
+        bool coop = false, tall = false;
+        for (int pass = 0; pass < 2; ++pass) {  // the second for CTAs with many rows
+            tall = pass == 1;
+            const int cap = hh_coop_capacity(tall), rows = tall ? 256 : hh_coop_rows();
+            coop = nh0 <= cap;
+            if (!coop) break;
             double tot = 0;
             for (auto& h : hh) tot += double(h.m);
             int used = 0;
+            int64_t most = 0;  // rows of a CTA
             for (auto& h : hh) {
                 h.ncta = std::max(1, int(double(cap - nh0) * double(h.m) / tot));
-                h.ncta = int(std::min<int64_t>(h.ncta, (h.m + hh_coop_rows() - 1) / hh_coop_rows()));
+                h.ncta = int(std::min<int64_t>(h.ncta, (h.m + rows - 1) / rows));
                 h.cta0 = used;
                 used += h.ncta;
+                most = std::max<int64_t>(most, h.m / h.ncta);
             }
             coop = used <= cap;
+            if (most <= hh_tall_rows()) break;
         }
         if (G.bars.bytes < hh.size() * sizeof(unsigned))
             G.bars.alloc(std::max<size_t>(hh.size() * sizeof(unsigned), 64), st);
@@ -1251,7 +1257,7 @@ void run_qr_move(TtnGroup& G, int v, int u, int maxdim, int mindim = 1, double c
             const int q0 = ctx->timer.mark();
             if (coop) {
                 TN_CUDA(cudaMemsetAsync(G.bars.p, 0, size_t(nh) * sizeof(unsigned), st));
-                launch_hh_panel_coop(dh, nh, nctas, p0, ctx->err.as<int>(), st);
+                launch_hh_panel_coop(dh, nh, nctas, tall, p0, ctx->err.as<int>(), st);
             } else {
                 for (int j = p0; j < std::min(pend, kmax); ++j)
                     launch_hh_column(dh, nh, mmax, j, p0, pend, st);

@@ -118,11 +118,12 @@ void launch_hh_finish(const HhDesc* d, int ninst, int64_t mnmax, cudaStream_t s)
 // -T of the whole block reflector from G = V^T V and the per-panel T (one CTA per instance)
 void launch_hh_tall(const HhDesc* d, int ninst, cudaStream_t s);
 // CTAs that the cooperative panel kernel may use (all co-resident on the device)
-int hh_coop_capacity();
+int hh_coop_capacity(bool tall);
+int hh_tall_rows();  // rows per CTA above which the panel takes the tall kernel
 int hh_coop_rows();  // rows of one of its CTAs in one pass
 // one panel [p0, p0 + HH_B) of every instance in one cooperative launch of nctas CTAs
 // (instance i owns CTAs [cta0, cta0 + ncta)); grid-wide waits are bounded and set *err
-void launch_hh_panel_coop(const HhDesc* d, int ninst, int nctas, int p0, int* err,
+void launch_hh_panel_coop(const HhDesc* d, int ninst, int nctas, bool tall, int p0, int* err,
                           cudaStream_t s);
 
 }  // namespace tn
