@@ -791,10 +791,19 @@ __device__ __forceinline__ Turn bj32_turn(float a, float b, float g, float tol) 
     const float ra = rsqrtf(a), rb = rsqrtf(b), cosine = g * ra * rb;
     if (!(fabsf(cosine) > tol)) return r;
     // tan = h / (d + sign(d) sqrt(d^2 + h^2)) with d = b - a and h = 2 g, both over sqrt(a b)
-    // (d stays below 1e19, h within [2 tol, 2]: no overflow of the squares)
     const float d = (b - a) * ra * rb, h = 2.f * cosine;
     const float w = fmaf(d, d, h * h);
-    const float t = __fdividef(h, d + copysignf(w * rsqrtf(w), d));
+    float t;
+    if (w <= 3.0e38f) {
+        t = __fdividef(h, d + copysignf(w * rsqrtf(w), d));
+    } else {
+        // the squares overflow where the norms differ by more than 2^64 (a column near the 1e-36
+        // bound beside one of a flat block, whose squared norm reaches the number of entries):
+        // there the tangent by the ratio, as bj_kernel forms it, and no turn that is a no-op
+        const float zeta = (b - a) / (2.f * g), az = fabsf(zeta);
+        t = az > 1e15f ? 0.5f / zeta : copysignf(1.f, zeta) / (az + sqrtf(1.f + zeta * zeta));
+        if (!isfinite(t) || t == 0.f) return r;
+    }
     const float c = rsqrtf(fmaf(t, t, 1.f));
     return Turn{c, c * t, t, true};
 }
