@@ -793,16 +793,13 @@ __device__ __forceinline__ Turn bj32_turn(float a, float b, float g, float tol) 
     // tan = h / (d + sign(d) sqrt(d^2 + h^2)) with d = b - a and h = 2 g, both over sqrt(a b)
     const float d = (b - a) * ra * rb, h = 2.f * cosine;
     const float w = fmaf(d, d, h * h);
-    float t;
-    if (w <= 3.0e38f) {
-        t = __fdividef(h, d + copysignf(w * rsqrtf(w), d));
-    } else {
+    float t = __fdividef(h, d + copysignf(w * rsqrtf(w), d));
+    if (!(w <= 3.0e38f)) {
         // the squares overflow where the norms differ by more than 2^64 (a column near the 1e-36
         // bound beside one of a flat block, whose squared norm reaches the number of entries):
-        // there the tangent by the ratio, as bj_kernel forms it, and no turn that is a no-op
-        const float zeta = (b - a) / (2.f * g), az = fabsf(zeta);
-        t = az > 1e15f ? 0.5f / zeta : copysignf(1.f, zeta) / (az + sqrtf(1.f + zeta * zeta));
-        if (!isfinite(t) || t == 0.f) return r;
+        // h^2 is nothing beside d^2 there
+        if (!(fabsf(h) < fabsf(d))) return r;
+        t = 0.5f * __fdividef(h, d);
     }
     const float c = rsqrtf(fmaf(t, t, 1.f));
     return Turn{c, c * t, t, true};
