@@ -1104,8 +1104,7 @@ template <class T, int B>
 void bj_launch(const BjDesc* d, int nd, int nctas, int maxn, float tol, int max_sweeps,
                int use_maxcos, int* err, cudaStream_t s) {
     const size_t shm = bj_smem<T, B>(maxn);
-    TN_CUDA(cudaFuncSetAttribute(bj_kernel<T, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(shm)));
+    allow_smem<bj_kernel<T, B>>(SMEM_MAX);
     void* args[] = {(void*)&d, (void*)&nd, (void*)&tol, (void*)&max_sweeps, (void*)&use_maxcos,
                     (void*)&err};
     TN_CUDA(cudaLaunchCooperativeKernel((const void*)bj_kernel<T, B>, dim3(nctas), dim3(BT), args,
@@ -1115,8 +1114,7 @@ void bj_launch(const BjDesc* d, int nd, int nctas, int maxn, float tol, int max_
 template <class T, int B>
 int bj_capacity(int maxn) {
     const size_t shm = bj_smem<T, B>(maxn);
-    TN_CUDA(cudaFuncSetAttribute(bj_kernel<T, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(shm)));
+    allow_smem<bj_kernel<T, B>>(SMEM_MAX);
     int dev = 0, nsm = 0, per = 0;
     TN_CUDA(cudaGetDevice(&dev));
     TN_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1173,8 +1171,7 @@ void launch_bsvd_panel(const BsvdBlk* d, int nb, int p0, int pw, int rmax, doubl
     if (nb <= 0) return;
     const size_t shm = size_t(rmax) * pw * 8;  // the panel rows of the tallest block
     TN_REQUIRE(pw >= 1 && pw <= 32 && shm <= size_t(PANEL_SMEM), "block SVD: panel too large");
-    TN_CUDA(cudaFuncSetAttribute(bsvd_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(shm)));
+    allow_smem<bsvd_panel_kernel>(PANEL_SMEM);
     bsvd_panel_kernel<<<nb, BT, shm, s>>>(d, ar, p0, pw);
     TN_CUDA(cudaGetLastError());
     count_launch();
@@ -1194,8 +1191,7 @@ int bsvd_jacobi_block(int maxn, int precision) {
 int bsvd_jacobi_capacity(int maxn, int precision) {
     if (use_bj32(maxn, precision)) {
         const size_t shm = bj32_smem(maxn);
-        TN_CUDA(cudaFuncSetAttribute(bj32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(shm)));
+        allow_smem<bj32_kernel>(bj32_smem(BJ32_MAXN));
         int dev = 0, nsm = 0, per = 0;
         TN_CUDA(cudaGetDevice(&dev));
         TN_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1221,8 +1217,7 @@ void launch_bsvd_jacobi(const BjDesc* d, int nd, int nctas, int maxn, int precis
     const float tdf = 3.55e-15f * sqrtf(float(maxn > 1 ? maxn : 1)) * 32.f;
     if (use_bj32(maxn, precision)) {
         const size_t shm = bj32_smem(maxn);
-        TN_CUDA(cudaFuncSetAttribute(bj32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(shm)));
+        allow_smem<bj32_kernel>(bj32_smem(BJ32_MAXN));
         float tol = 2.0e-5f;
         int max_sweeps = 30;
         void* args[] = {(void*)&d, (void*)&nd, (void*)&tol, (void*)&max_sweeps, (void*)&err};
@@ -1247,8 +1242,7 @@ void launch_bsvd_finish(const BsvdBlk* d, int nb, double* ar, double* qv, double
                         int* perm, cudaStream_t s) {
     if (nb <= 0) return;
     const size_t shm = size_t(bsvd_max_n()) * 8;
-    TN_CUDA(cudaFuncSetAttribute(bsvd_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(shm)));
+    allow_smem<bsvd_finish_kernel>(shm);
     bsvd_finish_kernel<<<nb, BT, shm, s>>>(d, ar, qv, py, S, perm);
     TN_CUDA(cudaGetLastError());
     bsvd_outputs_kernel<<<dim3(64, nb), 256, 0, s>>>(d, ar, qv, py);

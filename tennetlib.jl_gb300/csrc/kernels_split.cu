@@ -30,7 +30,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <type_traits>
 
 #include "tn_internal.h"
@@ -762,13 +761,10 @@ void launch_split_gemm(const SplitItem* items, int nitems, const SplitTask* task
                    : slices == 5 ? split_gemm_kernel<5>
                    : slices == 6 ? split_gemm_kernel<6>
                                  : split_gemm_kernel<7>;
-    static std::atomic<bool> attr[8][64];  // per device: the attribute belongs to its context
-    int dev = 0;
-    TN_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !attr[slices][dev]) {
-        TN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
-        if (dev >= 0 && dev < 64) attr[slices][dev] = true;
-    }
+    if (slices == 4) allow_smem<split_gemm_kernel<4>>(shm);
+    else if (slices == 5) allow_smem<split_gemm_kernel<5>>(shm);
+    else if (slices == 6) allow_smem<split_gemm_kernel<6>>(shm);
+    else allow_smem<split_gemm_kernel<7>>(shm);
     const int grid = nitems < nsm ? nitems : nsm;
     kernel<<<grid, THREADS, shm, s>>>(items, nitems, tasks, apack, bpack, ea, eb, b, err);
     TN_CUDA(cudaGetLastError());

@@ -1350,8 +1350,7 @@ void launch_svd_jacobi(const SvdBlockDesc* d, int nb, int max_n, const double* s
     if (max_n <= FAST_N) region = std::max<int64_t>(region, fast_smem(max_n));
     if (region + aux > limit) region = ((limit - aux) / 16) * 16;  // smaller blocks still fit
     const size_t shm = size_t(region + aux);
-    TN_CUDA(cudaFuncSetAttribute(svd_qrj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(shm)));
+    allow_smem<svd_qrj_kernel>(size_t(limit));
     svd_qrj_kernel<<<nb, SVD_THREADS, shm, s>>>(d, src, X, W, V, P, S, perm, sweeps_out,
                                                 int(region));
     TN_CUDA(cudaGetLastError());

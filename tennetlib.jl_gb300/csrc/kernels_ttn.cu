@@ -218,6 +218,7 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // Up to QC_ROWS rows of a lane are fetched side by side and stay in registers between the sum and
 // the update.
 constexpr int QC_CL = 8, QC_WARPS = BT / 32, QC_ROWS = 8;
+constexpr size_t QC_SMEM = size_t(200) * 1024;  // most shared memory of one of its CTAs
 
 // c -= tau v (v^T c) on the rows j and below: v is v[j + 1..m), 1 in row j; diag marks the lane of
 // row j, i0 is this lane's first row below it
@@ -1081,9 +1082,8 @@ size_t qr_cluster_smem(int64_t m, int64_t n) {
 // shm: the largest qr_cluster_smem of the matrices
 void launch_qr_small(const QrDesc* d, int ninst, size_t shm, cudaStream_t s) {
     if (ninst <= 0) return;
-    if (shm <= size_t(200) * 1024) {
-        TN_CUDA(cudaFuncSetAttribute(qr_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(shm)));
+    if (shm <= QC_SMEM) {
+        allow_smem<qr_cluster_kernel>(QC_SMEM);
         qr_cluster_kernel<<<ninst * QC_CL, BT, shm, s>>>(d);
     } else {
         qr_small_kernel<<<ninst, 1024, 0, s>>>(d);

@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 #include <stdexcept>
@@ -58,6 +59,22 @@ struct DevBuf {
     double* d() const { return static_cast<double*>(p); }
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
+
+// Opts a kernel in to `bytes` of dynamic shared memory: the most that any of its launches asks
+// for, once per device.  The attribute belongs to the kernel on the device and not to a context
+// or stream; set to the size of each launch, one host thread lowers it between the setting and
+// the launch of another, and that launch is refused.
+template <auto Kernel>
+void allow_smem(size_t bytes) {
+    constexpr int MAXDEV = 64;
+    static std::atomic<bool> done[MAXDEV];
+    int dev = 0;
+    TN_CUDA(cudaGetDevice(&dev));
+    const bool known = dev >= 0 && dev < MAXDEV;
+    if (known && done[dev]) return;
+    TN_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+    if (known) done[dev] = true;
+}
 
 // The tables of a plan in one device buffer: collected on the host, one allocation and one copy
 // (the host's side is kept with the plan: the copy may still be reading it).
