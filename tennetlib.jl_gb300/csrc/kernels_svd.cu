@@ -239,7 +239,10 @@ __host__ __device__ constexpr int fast_smem(int n) {
     return df > f32 ? df : f32;
 }
 
-struct FastShared {
+// (behind the matrices, in the dynamic part: as a static variable it took 4.7 KB from every
+// launch, and the Jacobi matrices of 118 and 119 columns, which need all but 4.3 and 0.5 KB, fell
+// back to global memory: 6.3 -> 10.0 and 6.4 -> 10.4 ms)
+struct alignas(16) FastShared {
     float cnf[FAST_N];           // column norms of the pivoting, by column
     int cp[FAST_N];              // column at a position
     df2 tau[FAST_N], h[FAST_N];
@@ -914,8 +917,8 @@ svd_qrj_kernel(const SvdBlockDesc* __restrict__ desc, const double* __restrict__
         if (clk && threadIdx.x == 0) clk[i] = clock64();
     };
     stamp(0);
-    if (m <= FAST_M && n <= FAST_N && fast_smem(n) <= smem_region) {
-        __shared__ FastShared sh;
+    if (m <= FAST_M && n <= FAST_N && fast_smem(n) + int(sizeof(FastShared)) <= smem_region) {
+        FastShared& sh = *reinterpret_cast<FastShared*>(smem + fast_smem(n));
         const int rm = (m + 31) / 32;
         if (warp >= fast_warps(rm)) return;  // these blocks synchronise through a barrier of W warps
         auto run = [&](auto cls, auto rows) {
@@ -1343,11 +1346,12 @@ void launch_svd_jacobi(const SvdBlockDesc* d, int nb, int max_n, const double* s
                        double* W, double* V, double* P, double* S, int* perm, int* sweeps_out,
                        cudaStream_t s) {
     if (nb <= 0) return;
-    const int64_t limit = 227 * 1024 - 2048 - int64_t(sizeof(FastShared));
+    const int64_t limit = 227 * 1024 - 2048;
     const int64_t aux = int64_t(max_n > 0 ? max_n : 1) * (3 * 8 + 4) + 16;
     TN_REQUIRE(aux < 96 * 1024, "SVD block too large (more than 3000 columns)");
     int64_t region = int64_t(2) * max_n * max_n * 8;
-    if (max_n <= FAST_N) region = std::max<int64_t>(region, fast_smem(max_n));
+    // room for the size classes of the blocks up to max_n
+    region = std::max<int64_t>(region, fast_smem(std::min(max_n, FAST_N)) + sizeof(FastShared));
     if (region + aux > limit) region = ((limit - aux) / 16) * 16;  // smaller blocks still fit
     const size_t shm = size_t(region + aux);
     allow_smem<svd_qrj_kernel>(size_t(limit));
