@@ -214,7 +214,7 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // each warp applies all reflectors to its own.  Bound by the FP64 pipe (2 multiply-adds per clock
 // and SM: 2 m n^2 of them take one SM 0.55 ms at 256 x 64) and the chain of a column (two sums,
 // root and division, barrier), so it takes eight SMs and their pipes for each matrix: four 256 x 64
-// matrices 1220 -> 420 us, 16 columns 90 -> 59 us, 64 x 64 (all chain) 288 -> 316 us.
+// matrices 1220 -> 420 us, four 256 x 16 144 -> 101 us, four 64 x 64 (all chain) 682 -> 258 us.
 // Up to QC_ROWS rows of a lane are fetched side by side and stay in registers between the sum and
 // the update.
 constexpr int QC_CL = 8, QC_WARPS = BT / 32, QC_ROWS = 8;
@@ -334,7 +334,7 @@ qr_cluster_kernel(const QrDesc* __restrict__ descs) {
 }
 
 // The same by one CTA per matrix on global memory, for columns too long for the shared memory of
-// a cluster (qr_cluster_smem)
+// a cluster (qr_by_cluster)
 __global__ void __launch_bounds__(1024) qr_small_kernel(const QrDesc* __restrict__ descs) {
     __shared__ double red[33];
     __shared__ double sc[3];
@@ -1074,22 +1074,31 @@ void launch_concat(const ConcatDesc* d, int ninst, int64_t nmax, cudaStream_t s)
     count_launch();
 }
 
-size_t qr_cluster_smem(int64_t m, int64_t n) {
+static size_t qr_cluster_smem(int64_t m, int64_t n) {
     const int64_t nl = (n + QC_CL - 1) / QC_CL;
     return size_t((nl + QC_WARPS) * m + nl) * 8;
 }
 
-// shm: the largest qr_cluster_smem of the matrices
-void launch_qr_small(const QrDesc* d, int ninst, size_t shm, cudaStream_t s) {
-    if (ninst <= 0) return;
-    if (shm <= QC_SMEM) {
+// Whether a cluster takes the matrix: while its columns fit the shared memory
+bool qr_by_cluster(int64_t m, int64_t n) { return qr_cluster_smem(m, n) <= QC_SMEM; }
+
+// the first ncluster matrices by clusters, the others by one CTA each
+void launch_qr_small(const QrDesc* d, const std::vector<QrDesc>& host, int ncluster,
+                     cudaStream_t s) {
+    if (ncluster > 0) {
+        size_t shm = 0;
+        for (int i = 0; i < ncluster; ++i)
+            shm = std::max(shm, qr_cluster_smem(host[size_t(i)].m, host[size_t(i)].n));
         allow_smem<qr_cluster_kernel>(QC_SMEM);
-        qr_cluster_kernel<<<ninst * QC_CL, BT, shm, s>>>(d);
-    } else {
-        qr_small_kernel<<<ninst, 1024, 0, s>>>(d);
+        qr_cluster_kernel<<<ncluster * QC_CL, BT, shm, s>>>(d);
+        TN_CUDA(cudaGetLastError());
+        count_launch();
     }
-    TN_CUDA(cudaGetLastError());
-    count_launch();
+    if (int(host.size()) > ncluster) {
+        qr_small_kernel<<<int(host.size()) - ncluster, 1024, 0, s>>>(d + ncluster);
+        TN_CUDA(cudaGetLastError());
+        count_launch();
+    }
 }
 
 void launch_hh_column(const HhDesc* d, int ninst, int64_t mmax, int j, int p0, int pend,

@@ -1205,11 +1205,12 @@ void run_qr_move(TtnGroup& G, int v, int u, int maxdim, int mindim = 1, double c
                                 cudaMemcpyDeviceToDevice, st));
     }
     if (!small.empty()) {
+        // each matrix by its own shape, whatever the others of the group are
+        const auto split = std::stable_partition(
+            small.begin(), small.end(), [](const QrDesc& q) { return qr_by_cluster(q.m, q.n); });
         upload_descs(G, G.d_qr, small);
         const int q0 = G.ctx->timer.mark();
-        size_t shm = 0;
-        for (const QrDesc& q : small) shm = std::max(shm, qr_cluster_smem(q.m, q.n));
-        launch_qr_small(G.d_qr.as<QrDesc>(), int(small.size()), shm, st);
+        launch_qr_small(G.d_qr.as<QrDesc>(), small, int(split - small.begin()), st);
         G.ctx->timer.add(T_QRPANEL, q0, G.ctx->timer.mark());
     }
     // a truncating move changes the dimensions: its plan is built for this move only

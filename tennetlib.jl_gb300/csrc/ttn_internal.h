@@ -108,8 +108,11 @@ void launch_blincomb(const BLinDesc* d, int ninst, int64_t nmax, cudaStream_t s)
 void launch_permute(const PermDesc* d, int ninst, int64_t nmax, cudaStream_t s);
 // the direct sum of subspace expansion along one leg; nmax >= every P (D1 + D2) Q
 void launch_concat(const ConcatDesc* d, int ninst, int64_t nmax, cudaStream_t s);
-size_t qr_cluster_smem(int64_t m, int64_t n);
-void launch_qr_small(const QrDesc* d, int ninst, size_t shm, cudaStream_t s);
+// small QRs of the matrices d (host: the same on the host): the first ncluster of them, which
+// qr_by_cluster has to hold for, by a cluster of CTAs each
+bool qr_by_cluster(int64_t m, int64_t n);
+void launch_qr_small(const QrDesc* d, const std::vector<QrDesc>& host, int ncluster,
+                     cudaStream_t s);
 void launch_hh_column(const HhDesc* d, int ninst, int64_t mmax, int j, int p0, int pend,
                       cudaStream_t s);
 void launch_hh_panel_end(const HhDesc* d, int ninst, int64_t mmax, int p0, int pb,
