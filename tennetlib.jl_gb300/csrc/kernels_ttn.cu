@@ -214,7 +214,8 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // each warp applies all reflectors to its own.  Bound by the FP64 pipe (2 multiply-adds per clock
 // and SM: 2 m n^2 of them take one SM 0.55 ms at 256 x 64) and the chain of a column (two sums,
 // root and division, barrier), so it takes eight SMs and their pipes for each matrix: four 256 x 64
-// matrices 1220 -> 420 us, four 256 x 16 144 -> 101 us, four 64 x 64 (all chain) 682 -> 258 us.
+// matrices 1220 -> 420 us, four 256 x 16 144 -> 101 us, four 64 x 64 (all chain) 682 -> 258 us; long
+// narrow matrices are slower (qr_by_cluster).
 // Up to QC_ROWS rows of a lane are fetched side by side and stay in registers between the sum and
 // the update.
 constexpr int QC_CL = 8, QC_WARPS = BT / 32, QC_ROWS = 8;
@@ -333,8 +334,8 @@ qr_cluster_kernel(const QrDesc* __restrict__ descs) {
     cl.sync();  // the others may still read this CTA's columns
 }
 
-// The same by one CTA per matrix on global memory, for columns too long for the shared memory of
-// a cluster (qr_by_cluster)
+// The same by one CTA per matrix on global memory, for long narrow matrices and those that do not
+// fit the shared memory of a cluster (qr_by_cluster)
 __global__ void __launch_bounds__(1024) qr_small_kernel(const QrDesc* __restrict__ descs) {
     __shared__ double red[33];
     __shared__ double sc[3];
@@ -1079,8 +1080,15 @@ static size_t qr_cluster_smem(int64_t m, int64_t n) {
     return size_t((nl + QC_WARPS) * m + nl) * 8;
 }
 
-// Whether a cluster takes the matrix: while its columns fit the shared memory
-bool qr_by_cluster(int64_t m, int64_t n) { return qr_cluster_smem(m, n) <= QC_SMEM; }
+// Whether a cluster takes the matrix: while its columns fit the shared memory, and not the long
+// narrow ones, whose column is a warp's work there and that of 32 warps in the one-CTA kernel
+// (one matrix, us, cluster against one CTA: 256 x 4 27 / 33, 320 x 4 37 / 33, 384 x 12 113 / 108,
+// 512 x 16 181 / 203, 512 x 12 135 / 137, 640 x 16 215 / 199, 640 x 20 273 / 275, 900 x 18
+// 308 / 289, 2048 x 8 270 / 182, 64 x 64 246 / 682; of 32 matrices 2048 x 8 807 / 183, the
+// clusters with 150 KB a CTA being one per eight SMs).
+bool qr_by_cluster(int64_t m, int64_t n) {
+    return qr_cluster_smem(m, n) <= QC_SMEM && !(m > 256 && m >= 40 * n);
+}
 
 // the first ncluster matrices by clusters, the others by one CTA each
 void launch_qr_small(const QrDesc* d, const std::vector<QrDesc>& host, int ncluster,
