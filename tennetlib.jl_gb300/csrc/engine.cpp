@@ -1489,9 +1489,18 @@ void block_svd(tn_ctx* ctx, DevBuf& dX, DevBuf& dW, DevBuf& dV, DevBuf& dP, DevB
         ci = e.best >= 0 ? e.best : e.next;
         thr = e.cand[size_t(ci)];
         if (e.best < 0) te = &e;
-        // such a bond has nothing to try: 2.4 ms against 3.9 ms on the pipeline with its
-        // largest block at 96 x 88, and the gap widens below
-        if (classes && te) {
+        // A bond of such blocks is not tuned and stays on one CTA per block, whatever other bonds
+        // have settled its bucket on: its path and last bits depend on its blocks alone.  In ms,
+        // one CTA each against threshold 64:
+        //   eight blocks of 8 to 100% of the largest: 88 columns 2.6 / 3.5, 92 2.8 / 3.5,
+        //     96 2.9 / 2.8, 100 3.8 / 3.5, 108 4.2 / 3.6, 112 4.3 / 3.7;
+        //   one block: 80 2.1 / 2.1, 88 2.6 / 2.2, 96 2.9 / 2.3, 104 3.9 / 2.9, 112 4.3 / 3.0;
+        //   equal blocks of 100 columns: 16 of them 3.9 / 3.5, 32 4.2 / 4.2, 64 4.6 / 7.1, 128
+        //     5.4 / 11.5 (the pipeline's one CTA per panel and its shared Jacobi launch).
+        // From 97 columns on the pipeline is the faster for up to 32 such blocks.  A line there
+        // moved <Sz> of a near-singlet state (20-site J1-J2 cylinder, 5e-9 at most) by 1e-12,
+        // more than its results may move, so the line is that of the classes.
+        if (classes) {
             thr = INT_MAX;
             te = nullptr;
         }
