@@ -239,7 +239,7 @@ __host__ __device__ constexpr int fast_smem(int n) {
     return df > f32 ? df : f32;
 }
 
-// (behind the matrices, in the dynamic part: as a static variable it took 4.7 KB from every
+// (before the matrices, in the dynamic part: as a static variable it took 4.7 KB from every
 // launch, and the Jacobi matrices of 118 and 119 columns, which need all but 4.3 and 0.5 KB, fell
 // back to global memory: 6.3 -> 10.0 and 6.4 -> 10.4 ms)
 struct alignas(16) FastShared {
@@ -918,13 +918,13 @@ svd_qrj_kernel(const SvdBlockDesc* __restrict__ desc, const double* __restrict__
     };
     stamp(0);
     if (m <= FAST_M && n <= FAST_N && fast_smem(n) + int(sizeof(FastShared)) <= smem_region) {
-        FastShared& sh = *reinterpret_cast<FastShared*>(smem + fast_smem(n));
+        FastShared& sh = *reinterpret_cast<FastShared*>(smem);
         const int rm = (m + 31) / 32;
         if (warp >= fast_warps(rm)) return;  // these blocks synchronise through a barrier of W warps
         auto run = [&](auto cls, auto rows) {
             svd_fast<decltype(cls)::value, decltype(rows)::value>(
                 d, src + d.src_off, reinterpret_cast<df2*>(X + d.x_off), W_ + d.x_off, V + d.v_off,
-                S, perm, smem, sh, sweeps_out, stamp);
+                S, perm, smem + sizeof(FastShared), sh, sweeps_out, stamp);
         };
         // the class of n, at least rm - 1 (n <= m); fast_smem allows for it
         const bool full = fast_class(n) == rm;
