@@ -1234,6 +1234,11 @@ void run_qr_move(TtnGroup& G, int v, int u, int maxdim, int mindim = 1, double c
             for (auto& h : hh) {
                 h.ncta = std::max(1, int(double(cap - nh0) * double(h.m) / tot));
                 h.ncta = int(std::min<int64_t>(h.ncta, (h.m + rows - 1) / rows));
+                // a matrix's CTAs meet at one counter for every column: no more than one per SM
+                // while that leaves them at most 512 rows (one matrix, us a panel, two per SM
+                // against one: 16000 rows 547 / 444, 24000 757 / 517, 38000 791 / 521, 60000
+                // 967 / 844, 77000 988 / 931, 130000 1287 / 1364)
+                if (!tall && h.m <= int64_t(512) * G.ctx->nsm) h.ncta = std::min(h.ncta, G.ctx->nsm);
                 h.cta0 = used;
                 used += h.ncta;
                 most = std::max<int64_t>(most, h.m / h.ncta);
