@@ -229,7 +229,10 @@ void GemmPlan::prepare(cudaStream_t s) const {
     // launch takes at least the total over the SMs and at least its longest tile.  Small plans
     // are bound by the longest tile (a 90 x 45 block with k = 900: 64, 128 or 512 clocks per k
     // on 16 x 8, 16 x 16 or 32 x 32), large ones by the total, where 32 x 32 has fewer CTAs.
-    constexpr double SMS = 152.0, CTA = 1200.0;
+    int dev = 0, nsm = 0;
+    TN_CUDA(cudaGetDevice(&dev));
+    TN_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    constexpr double CTA = 1200.0;
     constexpr int TILES[3][2] = {{32, 32}, {16, 16}, {16, 8}};
     double best = -1.0;
     for (const auto& T : TILES) {
@@ -241,7 +244,7 @@ void GemmPlan::prepare(cudaStream_t s) const {
             ntile += double((t.m + T[0] - 1) / T[0]) * ((t.n + T[1] - 1) / T[1]);
             longest = std::max(longest, 64.0 * std::min(pm, T[0] / 16) * std::min(pn, T[1] / 8) * w[i]);
         }
-        const double est = std::max((total + CTA * ntile) / SMS, longest + CTA);
+        const double est = std::max((total + CTA * ntile) / nsm, longest + CTA);
         if (best < 0.0 || est < best) {
             best = est;
             tile_m = T[0];
