@@ -543,7 +543,32 @@ def run_ours(args, world, rank, local, pg):
             res["j1j2_chi2048"] = run_j1j2(tn, local, args)
         except Exception as e:  # an extra leg: report it, keep the headline line
             res["j1j2_chi2048"] = {"error": f"{type(e).__name__}: {e}"}
-    print(json.dumps(res), flush=True)
+    # every figure of every leg goes to stderr: with the schedules and the sweeps of the quench
+    # the line would be 25 KB, too long for readers of the last few KB of a log
+    print("details " + json.dumps(res), file=sys.stderr, flush=True)
+    print(json.dumps(headline(res)), flush=True)
+
+
+LEGS = ("fp64_compare", "vs_cpu", "ttn", "quench", "j1j2_chi2048")
+
+
+def headline(res):
+    """The printed line: the run's own keys whole, of the legs their numbers (six digits) and
+    errors, without notes, schedules and lists."""
+    def short(v):
+        return float(f"{v:.6g}") if isinstance(v, float) else v
+
+    def numbers(d):
+        out = {k: short(v) for k, v in d.items()
+               if isinstance(v, (bool, int, float)) or k in ("workload", "error")}
+        for k, v in d.items():
+            if isinstance(v, dict):
+                out[k] = {a: short(b) for a, b in v.items() if isinstance(b, (bool, int, float))}
+        return out
+
+    drop = ("svd_schedule", "svd_roofline", "krylov_hbm_note")
+    return {k: numbers(v) if k in LEGS and isinstance(v, dict) else v
+            for k, v in res.items() if k not in drop}
 
 
 # J1-J2 cylinder at chi = 2048: the 6 x 16 cylinder (Ly = 6 periodic, Lx = 16 open, 96 sites,
