@@ -19,7 +19,8 @@ namespace tn {
 // Bound by the FP64 pipe: a warp-wide DFMA holds its SM sub-partition for 64 clocks (measured:
 // 1.7 FMA per clock and SM with one warp per sub-partition, 2.0 at most; DMMA the same), so a
 // multiplication by padding costs as much as a real one, while loads, shared memory and issue
-// slots are nearly free.  Hence small tiles of 8 x 4 warp patches (patches outside the block
+// slots are nearly free (launches of a few us are bound by the latency of their loads: a 20-site
+// cylinder's 6 to 17 us launches have the pipe 8 to 17% active).  Hence small tiles of 8 x 4 warp patches (patches outside the block
 // are skipped), k taken to its exact end, the segments of a task run together into one k range
 // (four 4-long segments fill a 16-deep chunk), four warps so that every sub-partition works,
 // and the next chunk's loads in flight during the products.  Each output is one chain of fused

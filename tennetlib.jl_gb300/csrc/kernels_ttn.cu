@@ -211,11 +211,12 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // belongs to warp (k / QC_CL) % 8 there, row i to lane i % 32.  Per column j the owning warp forms
 // the reflector (it has just updated the column), one cluster barrier, and every warp applies it
 // to its own columns, reading v from the owner's shared memory.  The columns of Q need no barrier:
-// each warp applies all reflectors to its own.  Bound by the FP64 pipe (2 multiply-adds per clock
-// and SM: 2 m n^2 of them take one SM 0.55 ms at 256 x 64) and the chain of a column (two sums,
-// root and division, barrier), so it takes eight SMs and their pipes for each matrix: four 256 x 64
-// matrices 1220 -> 420 us, four 256 x 16 144 -> 101 us, four 64 x 64 (all chain) 682 -> 258 us; long
-// narrow matrices are slower (qr_by_cluster).
+// each warp applies all reflectors to its own.  Bound by the chain of a column (two sums, root and
+// division, barrier): on the small matrices of a 64-site tree (17 to 60 us) ncu counts waits at
+// barriers first by far and the FP64 pipe 3 to 6% active.  With more rows the pipe counts too (2
+// multiply-adds per clock and SM: 2 m n^2 of them take one SM 0.55 ms at 256 x 64), so eight SMs
+// work on each matrix: four 256 x 64 matrices 1220 -> 420 us, four 256 x 16 144 -> 101 us, four
+// 64 x 64 682 -> 258 us; long narrow matrices are slower (qr_by_cluster).
 // Up to QC_ROWS rows of a lane are fetched side by side and stay in registers between the sum and
 // the update.
 constexpr int QC_CL = 8, QC_WARPS = BT / 32, QC_ROWS = 8;
@@ -584,12 +585,11 @@ __device__ __forceinline__ bool inst_barrier(unsigned* bar, unsigned target, int
 // a CTA can only reuse a buffer after the next barrier, which every CTA reaches only once it
 // has read the totals of the previous column.
 //
-// Bound by the FP64 pipe and the chain of a column (sums, barrier, totals, root and divisions,
-// update), not by memory.  A warp-wide FP64 operation takes 64 clocks, so a thread works on 8
-// columns of one row (4 even column groups, one per sub-partition, x 2 groups of 32 rows per CTA),
-// warp sums
-// are merged (9 adds for 8 columns instead of 40), and the two divisions of the reflector go to
-// two warps.  With one row of 32 columns per thread and plain butterflies (160 adds) a panel of
+// Bound by the chain of a column (sums, barrier, totals, root and divisions, update) and the FP64
+// pipe, not by memory (four 4096 x 64 matrices: barrier waits the largest stall, pipe 42% active).
+// A warp-wide FP64 operation takes 64 clocks, so a thread works on 8 columns of one row (4 even
+// column groups, one per sub-partition, x 2 groups of 32 rows per CTA), warp sums are merged (9
+// adds for 8 columns instead of 40), and the two divisions of the reflector go to two warps.  With one row of 32 columns per thread and plain butterflies (160 adds) a panel of
 // four 4096 x 64 matrices took 658 us, now 315 (four 64-site trees at chi = 64: 751 -> 675 ms a sweep).
 constexpr int HP_COLS = 8, HP_CG = HH_B / HP_COLS, HP_RG = BT / 32 / HP_CG;
 constexpr int HP_ROWS = 32 * HP_RG;  // rows of a CTA in one pass
@@ -718,7 +718,10 @@ hh_panel_coop_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* e
 // once, and the adds of the sums spread over many rows, for CTAs of more than HP_TALL rows.  There
 // the panel is bound by memory and the FP64 pipe, not by the chain of a column: 32 trees with
 // matrices up to 65536 x 256 (about 3000 rows a CTA) took 5.6 s of panels a sweep with it, 7.7 s
-// with the other; at 54 rows a CTA (four 4096 x 64 matrices) the other takes 305 us, this 658.
+// with the other.  The line is where they meet, us a panel with the other and with this: one matrix,
+// 256 rows a CTA 986 / 1331, 700 1593 / 1702, 900 1965 / 1955, 1030 1890 / 1870, 1400 2775 / 2639,
+// 3000 6765 / 5899; four, 710 1405 / 1501, 1040 1796 / 1933, 1420 2584 / 2454; 32, 790 1200 / 1502,
+// 1010 1718 / 1712, 1150 1647 / 1806, 1580 2723 / 2616.
 __global__ void __launch_bounds__(BT, 2)
 hh_panel_tall_kernel(const HhDesc* __restrict__ descs, int ninst, int p0, int* err) {
     constexpr int W1 = HH_B + 1;
@@ -1124,11 +1127,11 @@ void launch_hh_column(const HhDesc* d, int ninst, int64_t mmax, int j, int p0, i
     count_launch(2);
 }
 
-// co-resident CTAs of the cooperative panel kernel on the current device (cached per device)
 int hh_coop_rows() { return HP_ROWS; }
 
 int hh_tall_rows() { return HP_TALL; }
 
+// co-resident CTAs of the cooperative panel kernel on the current device (cached per device)
 int hh_coop_capacity(bool tall) {
     constexpr int MAXDEV = 64;
     static int caps[2][MAXDEV] = {};
