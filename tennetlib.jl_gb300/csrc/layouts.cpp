@@ -210,6 +210,18 @@ void GemmPlan::add_seg(int abuf, int64_t aoff, int lda, int ta, int bbuf, int64_
     flops += 2.0 * double(t.m) * double(t.n) * double(k);
 }
 
+// SMs of the current device (looked up once: a plan is prepared for every bond)
+static int device_sms() {
+    constexpr int MAXDEV = 64;
+    static std::atomic<int> known[MAXDEV];
+    int dev = 0, n = 0;
+    TN_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < MAXDEV && (n = known[dev]) > 0) return n;
+    TN_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    if (dev >= 0 && dev < MAXDEV) known[dev] = n;
+    return n;
+}
+
 void GemmPlan::prepare(cudaStream_t s) const {
     if (tab.dev.p) return;
     std::vector<Tile> tiles;
@@ -229,9 +241,7 @@ void GemmPlan::prepare(cudaStream_t s) const {
     // launch takes at least the total over the SMs and at least its longest tile.  Small plans
     // are bound by the longest tile (a 90 x 45 block with k = 900: 64, 128 or 512 clocks per k
     // on 16 x 8, 16 x 16 or 32 x 32), large ones by the total, where 32 x 32 has fewer CTAs.
-    int dev = 0, nsm = 0;
-    TN_CUDA(cudaGetDevice(&dev));
-    TN_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    const int nsm = device_sms();
     constexpr double CTA = 1200.0;
     constexpr int TILES[3][2] = {{32, 32}, {16, 16}, {16, 8}};
     double best = -1.0;
